@@ -1878,10 +1878,10 @@ constexpr int kSpSeg = 4096;
 
 // The tiles may span many short planes (the radially coarsened grid holds its rings in the z slot):
 // every run of four voxels has its own plane, so four q values (two theta, two z), q = u0 q[z0] + u1
-// q[z1] combined per run before the voxels' theta weights, which sum to one in the stencil: up = qb + ra (qa - qb), one
-// weight a voxel in registers (two leave one CTA an SM, 0.35 instead of 0.24 ms). The q segment
-// staged per group is the flat range of coarse voxels that the tile's taps touch. A thread whose runs
-// are not such pairs reads its taps from global memory.
+// q[z1] combined per run before the voxels' theta weights, which sum to one in the stencil: up = qa + rb
+// (qb - qa), one weight a voxel in registers (two leave one CTA an SM, 0.35 instead of 0.24 ms). The q
+// segment staged per group is the flat range of coarse voxels that the tile's taps touch. A thread whose
+// runs are not such pairs reads its taps from global memory.
 // Bound: HBM (sysmat rows) and issue. 12,288 BF16 rows of 36,000 voxels from 25 x 90: 0.24 ms (3.7 TB/s)
 // against 1.23 ms for a thread per voxel gathering q from L2; from 100 x 90: 0.247 ms (5.4 TB/s)
 // against 0.266 ms for a tile per plane with two weights a voxel.
@@ -1920,7 +1920,7 @@ sparse_group_scatter_flat_kernel(const float* __restrict__ q, int64_t ldq, const
   // flat coarse voxels of run r: z0 taps in at0[r], z1 taps in at1[r], theta a low, theta b high (the
   // coarse grid fits shared memory, so an index fits 16 bits)
   uint32_t at0[kSpRuns], at1[kSpRuns];
-  float u0[kSpRuns], u1[kSpRuns], ra[kSpVox];
+  float u0[kSpRuns], u1[kSpRuns], rb[kSpVox];
   bool pair = true;
   if (tid < kScConsumers) {
     int mn = INT_MAX, mx = -1;
@@ -1930,7 +1930,7 @@ sparse_group_scatter_flat_kernel(const float* __restrict__ q, int64_t ldq, const
       at0[r] = at1[r] = 0;
       u0[r] = u1[r] = 0.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) ra[4 * r + i] = 0.f;
+      for (int i = 0; i < 4; ++i) rb[4 * r + i] = 0.f;
       if (j >= j_end) continue;
       const int zf = j / n_lf, lf = j - zf * n_lf;  // (planes hold whole runs)
       const int z0 = taps.zt[2 * zf], z1 = taps.zt[2 * zf + 1];
@@ -1942,19 +1942,19 @@ sparse_group_scatter_flat_kernel(const float* __restrict__ q, int64_t ldq, const
         const int v = 4 * r + i;
         const int t[2] = {taps.lt[2 * (lf + i)], taps.lt[2 * (lf + i) + 1]};
         const float w[2] = {taps.lwt[2 * (lf + i)], taps.lwt[2 * (lf + i) + 1]};
-        float wb = 0.f;
+        float wa = 0.f;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (a < 0) a = t[h];
           if (t[h] == a) {
-            ra[v] += w[h];
+            wa += w[h];
           } else {
             if (b < 0) b = t[h];
-            if (t[h] == b) wb += w[h];
+            if (t[h] == b) rb[v] += w[h];
             else pair = false;
           }
         }
-        if (ra[v] + wb != 1.f) pair = false;
+        if (wa + rb[v] != 1.f || !(rb[v] <= 0.75f)) pair = false;
       }
       if (b < 0) b = a;
       at0[r] = (uint32_t)(z0 * n_lc + a) | (uint32_t)(z0 * n_lc + b) << 16;
@@ -2020,12 +2020,14 @@ sparse_group_scatter_flat_kernel(const float* __restrict__ q, int64_t ldq, const
 #pragma unroll
     for (int v = 0; v < kSpVox; ++v) acc[v] = 0.f;
     bool bad = false;
-    // run r's voxels: acc += a * (qb + ra (qa - qb)), a voxel whose factor is 0 untouched
+    // run r's voxels: acc += a * (qa + rb (qb - qa)), a voxel whose factor is 0 untouched. From qa, whose
+    // weight is at least 1/4: exact on the coarse sample itself (rb = 0) and a few ulp elsewhere, however
+    // much larger the neighbour is; from qb a small qa was lost in its rounding.
     auto add_pair = [&](int r, const float (&a)[4], float qa, float qb) {
 #pragma unroll
       for (int i = 0; i < 4; i += 2) {
         const int v = 4 * r + i;
-        const float2 val = __ffma2_rn(make_float2(ra[v], ra[v + 1]), make_float2(qa - qb, qa - qb), make_float2(qb, qb));
+        const float2 val = __ffma2_rn(make_float2(rb[v], rb[v + 1]), make_float2(qb - qa, qb - qa), make_float2(qa, qa));
         const float2 nw = __ffma2_rn(make_float2(a[i], a[i + 1]), val, make_float2(acc[v], acc[v + 1]));
         if (val.x != 0.f) acc[v] = nw.x;
         if (val.y != 0.f) acc[v + 1] = nw.y;
