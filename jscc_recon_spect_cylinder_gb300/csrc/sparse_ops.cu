@@ -1289,24 +1289,14 @@ sparse_group_coef_bulk_kernel(SpRows<TC> rows, const int32_t* __restrict__ order
         }
       }
     };
-    // Chunk u of a staged row (row: column 0). Chunks below n_full hold four columns of every thread
-    // and are read without a test, so that the reads of a chunk's events are issued together.
+    // LOOSE, chunk u of a staged row (row: column 0). Chunks below n_full hold four columns of every
+    // thread and are read without a test, so that the reads of a chunk's events are issued together (the
+    // aligned form's 16-byte reads are few enough: there the same costs 1%).
     const int n_full = vc / (kBkEvents * 4);
     auto take = [&](const TC* row, int u, bool all, float (&v)[4]) {
-      if constexpr (LOOSE) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          v[e] = all || 4 * u + e < kn ? to_float(row[et + kBkEvents * (4 * u + e)]) : 0.f;
-      } else {
-        const int c = et * 4 + u * (kBkEvents * 4);
-        v[0] = v[1] = v[2] = v[3] = 0.f;
-        if (all || c < vc) smem4(row, c, v);
-        if (RAGGED && !all && c < vc && c + 4 > vc) {  // padding past the row (any value) must not reach a sum
-#pragma unroll
-          for (int e = 1; e < 4; ++e)
-            if (c + e >= vc) v[e] = 0.f;
-        }
-      }
+      for (int e = 0; e < 4; ++e)
+        v[e] = all || 4 * u + e < kn ? to_float(row[et + kBkEvents * (4 * u + e)]) : 0.f;
     };
     // f(u, all): the chunks of the row
     auto for_chunks = [&](auto f) {
@@ -1393,13 +1383,33 @@ sparse_group_coef_bulk_kernel(SpRows<TC> rows, const int32_t* __restrict__ order
         float4 acc[NE];
 #pragma unroll
         for (int k = 0; k < NE; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for_chunks([&](int u, auto all) {
-          float v[NE][4];
+        if constexpr (LOOSE) {
+          for_chunks([&](int u, auto all) {
+            float v[NE][4];
 #pragma unroll
-          for (int k = 0; k < NE; ++k) take(row(k), u, decltype(all)::value, v[k]);
+            for (int k = 0; k < NE; ++k) take(row(k), u, decltype(all)::value, v[k]);
 #pragma unroll
-          for (int k = 0; k < NE; ++k) ffma4(acc[k], v[k], bv[u]);
-        });
+            for (int k = 0; k < NE; ++k) ffma4(acc[k], v[k], bv[u]);
+          });
+        } else {
+#pragma unroll
+          for (int u = 0; u < kBkQ; ++u) {
+            const int c = et * 4 + u * (kBkEvents * 4);
+            if (c < vc) {
+#pragma unroll
+              for (int k = 0; k < NE; ++k) {
+                float v[4];
+                smem4(slot(sl[k]), c, v);
+                if (RAGGED && c + 4 > vc) {  // padding past the row (any value) must not reach the dot
+#pragma unroll
+                  for (int e = 1; e < 4; ++e)
+                    if (c + e >= vc) v[e] = 0.f;
+                }
+                ffma4(acc[k], v, bv[u]);
+              }
+            }
+          }
+        }
 #pragma unroll
         for (int k = 0; k < NE; ++k) {
           const float f = warp_sum((acc[k].x + acc[k].y) + (acc[k].z + acc[k].w));
@@ -1425,7 +1435,7 @@ sparse_group_coef_bulk_kernel(SpRows<TC> rows, const int32_t* __restrict__ order
         }
         // ---- q_g += c_i t_i over the chunk, events in order (an event with c_i = 0 adds nothing,
         // whatever its row holds)
-        if (MODE != 2) {
+        if constexpr (MODE != 2 && LOOSE) {
           float ck[NE];
           bool none = true, all_events = true;
 #pragma unroll
@@ -1451,6 +1461,22 @@ sparse_group_coef_bulk_kernel(SpRows<TC> rows, const int32_t* __restrict__ order
                   float v[4];
                   take(row(k), u, false, v);
                   ffma4s(qa[u], ck[k], v);
+                }
+              }
+            }
+          }
+        } else if constexpr (MODE != 2) {
+#pragma unroll
+          for (int k = 0; k < NE; ++k) {
+            const float ck = __shfl_sync(0xffffffffu, cl, k);
+            if (ck != 0.f) {
+#pragma unroll
+              for (int u = 0; u < kBkQ; ++u) {
+                const int c = et * 4 + u * (kBkEvents * 4);
+                if (c < vc) {
+                  float v[4];
+                  smem4(slot(sl[k]), c, v);
+                  ffma4s(qa[u], ck, v);
                 }
               }
             }
