@@ -1,8 +1,9 @@
 // Fused SC weight: forward projection, ratio and back-projection in one read of the rows.
 //
 // For one rotation (the image read directly or gathered into the rotated view first),
-// u = A^T (proj / max(A x, floor)) over the bins b of one call (or another row_ratio of proj and A x,
-// and A x itself)
+// u = A^T (proj / max(A x, floor)) over the bins b of one call (LOGLIK: any row_ratio of proj and A x,
+// and A x itself into f_out where it is given; compiled apart, as the choice stands between every batch's
+// exchange and its back-projection)
 // (get_weight_single, recon_osem_plane.py:28-30). The two-pass form reads every row twice
 // (forward, then back); here each row is read once:
 //   * a cluster of two CTAs (one per SM) takes a contiguous range of the call's rows; CTA h
@@ -73,7 +74,7 @@ struct FsRow<float> {
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-template <typename T, bool LOOSE>
+template <typename T, bool LOOSE, bool LOGLIK>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFsThreads, 1)
 sc_fused_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __restrict__ row_idx, int64_t n_bins,
                 int64_t V, int64_t split, const float* __restrict__ x, const float* __restrict__ proj,
@@ -338,9 +339,14 @@ sc_fused_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __restrict_
       float r_lane = 0.f;
       if (lane < NB) {
         const float theirs = xbuf[par * kFsMaxBatch + lane];
-        const float f = h == 0 ? mine + theirs : theirs + mine;
-        if (f_out != nullptr && h == 0 && warp == 0) f_out[(b0 + bs + lane) * ld_f] = f;
-        r_lane = row_ratio(y_lane, f, mode, floor_v);
+        float f = h == 0 ? mine + theirs : theirs + mine;
+        if constexpr (LOGLIK) {
+          if (f_out != nullptr && h == 0 && warp == 0) f_out[(b0 + bs + lane) * ld_f] = f;
+          r_lane = row_ratio(y_lane, f, mode, floor_v);
+        } else {
+          if (mode == kRatioFloor) f = fmaxf(f, floor_v);
+          r_lane = y_lane / f;
+        }
       }
       // ---- back-projection: acc += r_k * row_k over this thread's columns, rows in order
       if constexpr (LOOSE) {

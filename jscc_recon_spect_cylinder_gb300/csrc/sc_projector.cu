@@ -586,7 +586,10 @@ static int sc_one_view(const T* A, int64_t lda, const int64_t* row_idx, int64_t 
                        stages, batch, stride)));
         return cudaSuccess;
       };
-      JSCC_CUDA_CHECK(loose ? launch(sc_fused_kernel<T, true>) : launch(sc_fused_kernel<T, false>));
+      if (mode == kRatioLog || mode == kRatioLogMinus || fout != nullptr)
+        JSCC_CUDA_CHECK(loose ? launch(sc_fused_kernel<T, true, true>) : launch(sc_fused_kernel<T, false, true>));
+      else
+        JSCC_CUDA_CHECK(loose ? launch(sc_fused_kernel<T, true, false>) : launch(sc_fused_kernel<T, false, false>));
       JSCC_LAUNCH_CHECK();
       return launch_reduce_scatter(fs_part, p.ldx, (int)p.fs_clusters, 1, 1, rotinv, ld_rot, 0, V, has_scale, scale,
                                    weight, st);
