@@ -277,12 +277,13 @@ sc_views_forward_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __r
           for (int i = 0; i < TM; ++i) a[i] = an[i];
         }
       }
-      // the columns past the last whole unit row of the matrix, one a lane and turn
-      for (int c = full * W + lane; c - lane < len; c += 32) {
+      // the columns past the last whole unit row of the matrix, one a lane and turn (a lane past the end
+      // adds nothing: 0 times another lane's image value would be NaN where that is infinite)
+      for (int c = full * W + lane; c < len; c += 32) {
         float a[TM];
 #pragma unroll
-        for (int i = 0; i < TM; ++i) a[i] = c < len ? load_elem(rowp[i], c) : 0.f;
-        accumulate(xs + (c < len ? slot(c) : 0) * XS, a);
+        for (int i = 0; i < TM; ++i) a[i] = load_elem(rowp[i], c);
+        accumulate(xs + slot(c) * XS, a);
       }
 #pragma unroll
       for (int i = 0; i < TM; ++i) rowp[i] += len;
