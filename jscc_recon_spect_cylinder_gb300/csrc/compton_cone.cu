@@ -1264,7 +1264,7 @@ int jscc_sparse_build_rows(const float* records, const int32_t* row_id, int64_t 
   const ConeEvent* rec = reinterpret_cast<const ConeEvent*>(records);
   const ReduceMaps m{z_ptr, z_idx, z_w, l_ptr, l_idx, l_w, n_lo, n_li};
   auto launch = [&](auto kernel, auto eff) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kernel, JSCC_SPARSE_BUILD_MAX_COARSE * (int)sizeof(float));
     if (e != cudaSuccess) return e;
     JSCC_TIMED("sparse_build_rows", st,
                (kernel<<<(unsigned)n_ev, kBuildThreads, smem, st>>>(rec, row_id, coor, (int)vc, eff, ld_sysmat, m,

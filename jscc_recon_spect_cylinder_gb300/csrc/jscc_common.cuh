@@ -89,6 +89,15 @@ int launch_rows_weight(const float* A, int64_t lda, int64_t n_rows, int64_t V, c
                        const int64_t* rotinv, int64_t ld_rot, int mode, float floor_v, float scale, float* weight,
                        float* f_out, void* ws, size_t ws_bytes, cudaStream_t st);
 
+// The shared memory that a launch may ask for is a property of the kernel, shared by all threads of the
+// process: every launch sets the same value, the most that any call of the kernel needs, so that none
+// lowers another's.
+constexpr int kMaxDynamicSmem = 227 * 1024;
+template <typename K>
+inline cudaError_t allow_smem(K* kernel, int most = kMaxDynamicSmem) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Carves aligned sub-buffers out of a caller-provided workspace.

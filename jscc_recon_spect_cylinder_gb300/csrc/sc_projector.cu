@@ -578,7 +578,7 @@ static int sc_one_view(const T* A, int64_t lda, const int64_t* row_idx, int64_t 
     if (split <= kFsHalfMax && V - split <= kFsHalfMax && V - split > 0 && stages >= 2 && batch >= 1) {
       const size_t smem = kFsHeader + (size_t)stages * stride;
       auto launch = [&](auto kernel) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(kernel);
         if (e != cudaSuccess) return e;
         JSCC_TIMED("sc_fused", st,
                    (kernel<<<(unsigned)(2 * p.fs_clusters), kFsThreads, smem, st>>>(
@@ -611,7 +611,7 @@ static int sc_one_view(const T* A, int64_t lda, const int64_t* row_idx, int64_t 
     const bool smem_x = vec_ok && xbytes <= 200 * 1024;
     const unsigned grid = (unsigned)(G / 32);
     auto launch = [&](auto kernel, size_t sh) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+      cudaError_t e = allow_smem(kernel);
       if (e != cudaSuccess) return e;
       JSCC_TIMED("sc_forward_split", st,
                  (kernel<<<grid, 1024, sh, st>>>(A, lda, row_idx, n_bins, V, x, nvr, L, p.fwd_maxp, fpart)));

@@ -556,8 +556,7 @@ static int sv_launch_block(const T* A, int64_t lda, const int64_t* row_idx, int6
   using Tr = SvTraits<T, NB, RING>;
   if (stage != 2) {
     const size_t smem = Tr::kFwdRing + align_up((size_t)p.piece_cols * p.pitch * sizeof(float), 16);
-    JSCC_CUDA_CHECK(cudaFuncSetAttribute(sc_views_forward_kernel<T, NB, RING>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    JSCC_CUDA_CHECK(allow_smem(sc_views_forward_kernel<T, NB, RING>));
     JSCC_TIMED("sc_views_forward", st,
                (sc_views_forward_kernel<T, NB, RING><<<dim3((unsigned)p.slices, (unsigned)p.row_splits), kSvThreads,
                                                        smem, st>>>(A, lda, row_idx, n_bins, V, xt, p.slices,
@@ -572,7 +571,7 @@ static int sv_launch_block(const T* A, int64_t lda, const int64_t* row_idx, int6
   }
   const int64_t tiles = (V + kSvBackCols - 1) / kSvBackCols;
   auto back = [&](auto kernel, int smem) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem(kernel);
     if (e != cudaSuccess) return e;
     JSCC_TIMED("sc_views_back", st,
                (kernel<<<dim3((unsigned)tiles, (unsigned)p.chunks), kSvThreads, smem, st>>>(

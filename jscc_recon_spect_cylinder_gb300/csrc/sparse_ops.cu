@@ -2190,9 +2190,7 @@ static int cf_max_clusters(size_t smem) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   if (cache_dev[dev] > 0 && cache_smem[dev] == smem) return cache_dev[dev];
-  if (cudaFuncSetAttribute(sparse_cluster_fused_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return 0;
+  if (allow_smem(sparse_cluster_fused_kernel<MODE>) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(num_sms() / kCfCluster * kCfCluster));
   cfg.blockDim = dim3(kCfThreads);
@@ -2384,8 +2382,7 @@ static int grouped_launch(const SpRows<TC>& rows, bool vec_rows, int64_t n_event
   cudaError_t attr = cudaSuccess;
 #define JSCC_GA_Z(KZ, X)                                                                                         \
   do {                                                                                                           \
-    attr = cudaFuncSetAttribute(sparse_group_adjoint_zring_kernel<KZ, TE>,                                       \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)az_smem);                      \
+    attr = allow_smem(sparse_group_adjoint_zring_kernel<KZ, TE>);                                                \
     if (attr == cudaSuccess)                                                                                     \
       JSCC_TIMED("sparse_group_adjoint", st,                                                                     \
                  (sparse_group_adjoint_zring_kernel<KZ, TE><<<az, kAzThreads + 32, az_smem, st>>>(               \
@@ -2395,8 +2392,7 @@ static int grouped_launch(const SpRows<TC>& rows, bool vec_rows, int64_t n_event
 #define JSCC_GA(TP, XS, X)                                                                                       \
   do {                                                                                                           \
     if (ring) {                                                                                                  \
-      attr = cudaFuncSetAttribute(sparse_group_adjoint_ring_kernel<TE>,                                          \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ad_smem);                    \
+      attr = allow_smem(sparse_group_adjoint_ring_kernel<TE>);                                                   \
       if (attr == cudaSuccess)                                                                                   \
         JSCC_TIMED("sparse_group_adjoint", st,                                                                   \
                    (sparse_group_adjoint_ring_kernel<TE><<<dim3((unsigned)ad_tiles, (unsigned)ad_chunks),        \
@@ -2430,8 +2426,7 @@ static int grouped_launch(const SpRows<TC>& rows, bool vec_rows, int64_t n_event
 #define JSCC_GC_BK_K(MODE, RAGGED, LOOSE)                                                                        \
   do {                                                                                                           \
     if (attr == cudaSuccess)                                                                                     \
-      attr = cudaFuncSetAttribute(sparse_group_coef_bulk_kernel<MODE, TC, RAGGED, LOOSE>,                        \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bk_smem);                    \
+      attr = allow_smem(sparse_group_coef_bulk_kernel<MODE, TC, RAGGED, LOOSE>);                                 \
     if (attr == cudaSuccess)                                                                                     \
       JSCC_TIMED(MODE == 2 ? "sparse_group_rowsum" : "sparse_group_coef", st,                                    \
                  (sparse_group_coef_bulk_kernel<MODE, TC, RAGGED, LOOSE><<<(unsigned)bk_grid, kBkThreads,        \
@@ -2449,8 +2444,7 @@ static int grouped_launch(const SpRows<TC>& rows, bool vec_rows, int64_t n_event
   } while (0)
 #define JSCC_GC_K(MODE, KT, TW)                                                                                  \
   do {                                                                                                           \
-    attr = cudaFuncSetAttribute(sparse_group_coef_kernel<MODE, KT, TE, TC>,                                      \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                         \
+    attr = allow_smem(sparse_group_coef_kernel<MODE, KT, TE, TC>);                                               \
     if (attr == cudaSuccess)                                                                                     \
       JSCC_TIMED(MODE == 2 ? "sparse_group_rowsum" : "sparse_group_coef", st,                                    \
                  (sparse_group_coef_kernel<MODE, KT, TE, TC><<<(unsigned)grid, kGcThreads, smem, st>>>(          \
@@ -2602,8 +2596,7 @@ static int grouped_launch(const SpRows<TC>& rows, bool vec_rows, int64_t n_event
     if (sc_chunks > n_groups) sc_chunks = n_groups;
     if (sc_chunks < 1) sc_chunks = 1;
     const int sc_gpc = (int)((n_groups + sc_chunks - 1) / sc_chunks);
-    JSCC_CUDA_CHECK(cudaFuncSetAttribute(sparse_group_scatter_flat_kernel<TE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_smem));
+    JSCC_CUDA_CHECK(allow_smem(sparse_group_scatter_flat_kernel<TE>));
     JSCC_TIMED("sparse_group_scatter", st,
                (sparse_group_scatter_flat_kernel<TE><<<dim3((unsigned)tiles, (unsigned)sc_chunks), kScThreads,
                                                        sc_smem, st>>>(q, ldq, grow, n_groups, sc_gpc, eff, ld_eff,
@@ -2619,8 +2612,7 @@ static int grouped_launch(const SpRows<TC>& rows, bool vec_rows, int64_t n_event
     if (sc_chunks > n_groups) sc_chunks = n_groups;
     if (sc_chunks < 1) sc_chunks = 1;
     const int sc_gpc = (int)((n_groups + sc_chunks - 1) / sc_chunks);
-    JSCC_CUDA_CHECK(cudaFuncSetAttribute(sparse_group_scatter_bulk_kernel<TE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_smem));
+    JSCC_CUDA_CHECK(allow_smem(sparse_group_scatter_bulk_kernel<TE>));
     JSCC_TIMED("sparse_group_scatter", st,
                (sparse_group_scatter_bulk_kernel<TE><<<dim3((unsigned)tiles, (unsigned)sc_chunks), kScThreads,
                                                        sc_smem, st>>>(q, ldq, grow, n_groups, sc_gpc, eff, ld_eff,
