@@ -332,8 +332,10 @@ def sc_loglik(sysmat, proj, img, rotmat=None, rotmat_inv=None, eps=0.0):
     x = _f32_contig(img.reshape(-1))
     if x.numel() != n_vox:
         raise ValueError(f"img has {x.numel()} voxels, sysmat has {n_vox}")
-    if proj.dtype != torch.float32 or not proj.is_contiguous() or proj.shape != (n_bins, n_rot) or ld_rot != ld_inv:
-        raise ValueError("proj must be float32 [bins, rotations], the rotation tables alike")
+    if proj.dtype != torch.float32 or not proj.is_contiguous() or proj.shape != (n_bins, n_rot):
+        raise ValueError("proj must be float32 [bins, rotations]")
+    if rm is not None and ri is not None and ld_rot != ld_inv:  # the call takes one row pitch
+        rm, ri, ld_rot = rm[:, :n_rot].contiguous(), ri[:, :n_rot].contiguous(), n_rot
     f = torch.empty((n_bins, n_rot), dtype=torch.float32, device=dev)
     grad = torch.zeros((n_vox, 1), dtype=torch.float32, device=dev)
     lib = _lib.load()
