@@ -19,6 +19,7 @@ the gradient kept for backward), and map_reconstruct minimises
 from __future__ import annotations
 
 import torch
+from torch.autograd.function import once_differentiable
 
 from . import _lib, ops
 
@@ -66,7 +67,8 @@ def compton_project(x, events, coor, sysmat, use_window=False):
 
 
 class SCLogLik(torch.autograd.Function):
-    """sum_b (y_b log max(f_b, eps) - f_b) (float64 0-d); the forward pass computes the gradient too."""
+    """sum_b (y_b log max(f_b, eps) - f_b) (float64 0-d); the forward pass computes the gradient too.
+    Once differentiable: the saved gradient is a constant to autograd, a second derivative would lack it."""
 
     @staticmethod
     def forward(ctx, x, sysmat, y, rotmat, rotmat_inv, eps):
@@ -77,6 +79,7 @@ class SCLogLik(torch.autograd.Function):
         return (y.double() * torch.log(f.clamp_min(eps)) - f).sum()
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, gv):
         (grad,) = ctx.saved_tensors
         return (grad * gv).reshape(ctx.shape), None, None, None, None, None
@@ -92,6 +95,7 @@ class ComptonLogLik(torch.autograd.Function):
         return torch.log(g.double().clamp_min(eps)).sum()
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, gv):
         (grad,) = ctx.saved_tensors
         return (grad * gv).reshape(ctx.shape), None, None, None
