@@ -674,7 +674,9 @@ static int sc_run(const T* A, int64_t lda, const int64_t* row_idx, int64_t n_bin
                   size_t ws_bytes, cudaStream_t st, int stage, float* fout, int64_t ld_fout, const float* gin,
                   int64_t ld_gin) {
   const int has_scale = scale != 1.0f;
-  if (n_rot > 1 || one_view_by_views<T>(A, lda, n_bins, V, stage))
+  // (one view in less than its padding to two takes goes the way that the smallest workspace is made for)
+  if (n_rot > 1 || (one_view_by_views<T>(A, lda, n_bins, V, stage) &&
+                    plan_views(n_bins, V, 1, ws_bytes).bytes <= ws_bytes))
     return sc_views<T>(A, lda, row_idx, n_bins, V, proj, ld_proj, n_rot, img, rotmat, rotinv, ld_rot, mode,
                        floor_v, has_scale, scale, weight, ws, ws_bytes, st, stage, fout, ld_fout, gin, ld_gin);
   Carver cv(ws, ws_bytes);
