@@ -1070,8 +1070,11 @@ static ConePlan plan_cone(int64_t n_ev, int64_t V) {
   b += align_up((size_t)p.chunks * p.ldp * sizeof(float), 256);            // partials
   p.ws_bytes = b + 256;
   if (n_ev < 1 || V < 1) return p;
-  // the strict model's weight: rows of whole stages of events, as many as kConeStoreMax bytes hold
-  const int64_t fit = (int64_t)(kConeStoreMax / (sizeof(float) * (size_t)p.ldp)) / kRowsStage * kRowsStage;
+  // the strict model's weight: rows of whole stages of events, as many as kConeStoreMax bytes hold and
+  // one grid has (stages in its y: grids of at most 64 voxels meet that first)
+  int64_t stages = (int64_t)(kConeStoreMax / (sizeof(float) * (size_t)p.ldp)) / kRowsStage;
+  if (stages > 65535) stages = 65535;
+  const int64_t fit = stages * kRowsStage;
   p.store_ev = n_ev < fit ? n_ev : fit;
   if (p.store_ev > 0) {
     p.sc_bytes = rows_weight_bytes(p.store_ev, V);
