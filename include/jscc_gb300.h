@@ -286,6 +286,12 @@ JSCC_API int jscc_sparse_build_rows(const float* records, const int32_t* row_id,
  * vectors and the partial images, the passes evaluate every pair themselves. */
 JSCC_API size_t jscc_compton_weight_workspace_bytes(int64_t n_ev, int64_t n_vox);
 
+/* Workspace of one of them alone: call 0 jscc_compton_weight, 1 jscc_compton_project, 2
+ * jscc_compton_backproject, with its model and use_window. preferred != 0: with the room for rows or slices,
+ * where the call has use for either (a strict model, no window); 0: the least that it takes. */
+JSCC_API size_t jscc_compton_workspace_bytes(int64_t n_ev, int64_t n_vox, int32_t call, int32_t model,
+                   int32_t use_window, int32_t preferred);
+
 /*
  * Fused list-mode Compton weight with T recomputed on the fly (never stored):
  *   x_r = img[rotmat[:, 0] - 1]            (identity when rotmat == NULL)

@@ -174,6 +174,7 @@ _SIGNATURES: dict[str, tuple] = {
         [c_void_p, c_int32, c_int64, c_int64, c_int64, c_void_p, c_int64, c_int32, c_void_p, c_void_p, c_void_p,
          c_int64, c_float, c_void_p, c_int64, c_void_p, c_void_p, c_size_t, c_void_p],
     ),
+    "jscc_compton_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int32, c_int32, c_int32, c_int32]),
     "jscc_compton_loglik_workspace_bytes": (c_size_t, [c_int64, c_int64]),
     "jscc_compton_loglik": (
         c_int,
@@ -392,25 +393,41 @@ class _Workspace:
 
     def __init__(self) -> None:
         self._bufs: dict[tuple[int, int], torch.Tensor] = {}
+        self._refused: dict[tuple[int, int], int] = {}
         self._captured: set[tuple[int, int]] = set()
         self._kept: list[torch.Tensor] = []
 
-    def get(self, device: torch.device, nbytes: int) -> torch.Tensor:
+    def get(self, device: torch.device, nbytes: int, at_least: int | None = None) -> torch.Tensor:
+        """At least ``nbytes`` of scratch; where they cannot be had and the caller can work in less,
+        ``at_least`` of them (a request that failed is not tried again before ``clear``: each trial
+        would wait for the device and empty torch's cache)."""
         key = (device.index if device.index is not None else torch.cuda.current_device(),
                stream_handle(device))
         if key not in self._captured and torch.cuda.is_current_stream_capturing():
             self._captured.add(key)
         buf = self._bufs.get(key)
-        if buf is None or buf.numel() < nbytes:
-            if buf is not None and key in self._captured:
-                self._kept.append(buf)
-                nbytes = max(nbytes, buf.numel() * 3 // 2)
-            buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
-            self._bufs[key] = buf
-        return buf
+        if at_least is not None and nbytes >= self._refused.get(key, nbytes + 1):
+            nbytes = at_least
+        if buf is not None and buf.numel() >= nbytes:
+            return buf
+        size = nbytes
+        if buf is not None and key in self._captured:
+            size = max(nbytes, buf.numel() * 3 // 2)
+        try:
+            new = torch.empty(max(size, 256), dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            if at_least is None or at_least >= nbytes:
+                raise
+            self._refused[key] = nbytes
+            return self.get(device, at_least)
+        if buf is not None and key in self._captured:
+            self._kept.append(buf)
+        self._bufs[key] = new
+        return new
 
     def clear(self) -> None:
         self._bufs.clear()
+        self._refused.clear()
         self._captured.clear()
         self._kept.clear()
 

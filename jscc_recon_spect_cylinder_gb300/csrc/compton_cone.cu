@@ -1044,7 +1044,8 @@ struct ConePlan {
   int slices;           // the strict projection's voxel slices
   int64_t store_ev;     // events whose rows the weight stores at a time
   size_t sc_bytes;      // workspace of the SC kernels over them
-  size_t more_bytes;    // workspace beyond the minimum for the stored rows, or the slices' sums
+  size_t store_bytes;   // workspace beyond the minimum for the stored rows
+  size_t slice_bytes;   // and for the slices' sums
 };
 
 constexpr int kConeFwdCtas = 5;                       // resident forward CTAs an SM
@@ -1078,15 +1079,14 @@ static ConePlan plan_cone(int64_t n_ev, int64_t V) {
   p.store_ev = n_ev < fit ? n_ev : fit;
   if (p.store_ev > 0) {
     p.sc_bytes = rows_weight_bytes(p.store_ev, V);
-    p.more_bytes = align_up((size_t)p.store_ev * p.ldp * sizeof(float), 256) + align_up(p.sc_bytes, 256) + 512;
+    p.store_bytes = align_up((size_t)p.store_ev * p.ldp * sizeof(float), 256) + align_up(p.sc_bytes, 256) + 512;
   }
   // the strict projection: slices of at least eight voxels a thread until two waves of CTAs run
   const int64_t n_blocks = (n_ev + 15) / 16;
   int64_t slices = 2 * (int64_t)kConeFwdCtas * num_sms() / n_blocks;
   if (slices > V / (8 * kConeThreads)) slices = V / (8 * kConeThreads);
   p.slices = (int)(slices < 1 ? 1 : (slices > 16 ? 16 : slices));
-  const size_t fs = align_up((size_t)p.slices * n_ev * sizeof(float), 256) + 256;
-  if (p.slices > 1 && p.more_bytes < fs) p.more_bytes = fs;
+  if (p.slices > 1) p.slice_bytes = align_up((size_t)p.slices * n_ev * sizeof(float), 256) + 256;
   return p;
 }
 
@@ -1149,7 +1149,7 @@ static int launch_cone_stored(const ConeEvent* rec, const int32_t* rid, int64_t 
                               const float* x, const TE* eff, int64_t ld_eff, const int64_t* rotinv, int64_t ld_rot,
                               int mode, float floor_v, float scale, float* weight, float* f, const ConePlan& p,
                               void* more, cudaStream_t st) {
-  Carver cv(more, p.more_bytes);
+  Carver cv(more, p.store_bytes);
   float* rows = cv.take<float>((size_t)p.store_ev * p.ldp);
   float* one = cv.take<float>(1);
   char* sc = cv.take<char>(p.sc_bytes);
@@ -1323,7 +1323,20 @@ int jscc_compton_row_stats(const float* records, const int32_t* row_id, int64_t 
 
 size_t jscc_compton_weight_workspace_bytes(int64_t n_ev, int64_t n_vox) {
   const ConePlan p = plan_cone(n_ev, n_vox);
-  return p.ws_bytes + p.more_bytes;
+  return p.ws_bytes + (p.store_bytes > p.slice_bytes ? p.store_bytes : p.slice_bytes);
+}
+
+// What a call uses beyond the minimum: the strict weight over every pair stores rows, the strict
+// projection over every pair has slices; nothing else does either.
+static size_t cone_more_bytes(const ConePlan& p, int stage, int32_t model, int32_t use_window) {
+  if (model != JSCC_CONE_STRICT || use_window) return 0;
+  return stage == 0 ? p.store_bytes : stage == 1 ? p.slice_bytes : 0;
+}
+
+size_t jscc_compton_workspace_bytes(int64_t n_ev, int64_t n_vox, int32_t call, int32_t model, int32_t use_window,
+                                    int32_t preferred) {
+  const ConePlan p = plan_cone(n_ev, n_vox);
+  return p.ws_bytes + (preferred ? cone_more_bytes(p, call, model, use_window) : 0);
 }
 
 // The weight and its two halves (the differentiable projector's forward and backward):
@@ -1358,7 +1371,8 @@ static int compton_stage_entry(const char* what, int stage, const float* records
   JSCC_REQUIRE(cv.ok(), "%s: workspace carve overflow", what);
   // with less than the plan's workspace the weight's passes each evaluate every pair
   const size_t at = align_up(cv.off, 256);
-  void* more = p.more_bytes > 0 && at + p.more_bytes <= workspace_bytes ? static_cast<char*>(workspace) + at : nullptr;
+  const size_t more_bytes = cone_more_bytes(p, stage, model, use_window);
+  void* more = more_bytes > 0 && at + more_bytes <= workspace_bytes ? static_cast<char*>(workspace) + at : nullptr;
   if (stage == 1) f = f_out;
   if (stage == 2) q = const_cast<float*>(g);  // read only by the back kernel
   cudaStream_t st = as_stream(stream);
@@ -1422,7 +1436,7 @@ int jscc_compton_weight(const float* records, const int32_t* row_id, int64_t n_e
 
 size_t jscc_compton_loglik_workspace_bytes(int64_t n_ev, int64_t n_vox) {
   const ConePlan p = plan_cone(n_ev, n_vox);
-  return p.store_ev > 0 ? p.more_bytes : 0;
+  return p.store_bytes;
 }
 
 int jscc_compton_loglik(const float* records, const int32_t* row_id, int64_t n_ev, const float* coor, int64_t n_vox,
@@ -1436,8 +1450,8 @@ int jscc_compton_loglik(const float* records, const int32_t* row_id, int64_t n_e
   JSCC_REQUIRE(!eff || ld_eff >= n_vox, "%s: efficiency rows need ld >= V", what);
   const ConePlan p = plan_cone(n_ev, n_vox);
   JSCC_REQUIRE(p.store_ev > 0, "%s: too many voxels (%lld)", what, (long long)n_vox);
-  JSCC_REQUIRE(workspace && workspace_bytes >= p.more_bytes, "%s: workspace too small (%zu < %zu)", what,
-               workspace_bytes, p.more_bytes);
+  JSCC_REQUIRE(workspace && workspace_bytes >= p.store_bytes, "%s: workspace too small (%zu < %zu)", what,
+               workspace_bytes, p.store_bytes);
   const ConeEvent* rec = reinterpret_cast<const ConeEvent*>(records);
   cudaStream_t st = as_stream(stream);
   return eff_dtype == JSCC_DTYPE_F32

@@ -233,6 +233,13 @@ def sc_backproject(sysmat, g, rotmat_inv=None, n_rot=None, row_idx=None, scale=1
     return out
 
 
+def _compton_scratch(lib, dev, n, V, call, model, use_window):
+    """Scratch of a Compton call (0 weight, 1 project, 2 backproject): what it prefers (the strict weight:
+    up to 1 GB of rows), or the least it takes where memory is short."""
+    want, least = (lib.jscc_compton_workspace_bytes(n, V, call, int(model), 1 if use_window else 0, p) for p in (1, 0))
+    return _lib.workspace.get(dev, want, least)
+
+
 def compton_project(records, row_id, coor, img, model=_lib.CONE_STRICT, eff=None, use_window=False, rotmat=None,
                     rot_col=0):
     """Forward list-mode projection ``f[i] = sum_j t_ij rot(img)_j`` with T recomputed
@@ -264,7 +271,7 @@ def compton_project(records, row_id, coor, img, model=_lib.CONE_STRICT, eff=None
         records, row_id, perm = _row_sorted_events(records, row_id)
     f = torch.empty(n, dtype=torch.float32, device=dev)
     lib = _lib.load()
-    ws = _lib.workspace.get(dev, lib.jscc_compton_weight_workspace_bytes(n, V))
+    ws = _compton_scratch(lib, dev, n, V, 1, model, use_window)
     rc = lib.jscc_compton_project(records.data_ptr(), row_id.data_ptr(), n, c.data_ptr(), V, int(model),
                                   1 if use_window else 0, _lib.ptr(e), edt, ld, x.data_ptr(),
                                   None if rm is None else rm.data_ptr() + rot_col * 8, 0 if rm is None else rm.stride(0),
@@ -310,7 +317,7 @@ def compton_backproject(records, row_id, coor, g, model=_lib.CONE_STRICT, eff=No
     if out is None:
         out = torch.zeros((V, 1), dtype=torch.float32, device=dev)
     lib = _lib.load()
-    ws = _lib.workspace.get(dev, lib.jscc_compton_weight_workspace_bytes(n, V))
+    ws = _compton_scratch(lib, dev, n, V, 2, model, use_window)
     rc = lib.jscc_compton_backproject(records.data_ptr(), row_id.data_ptr(), n, c.data_ptr(), V, int(model),
                                       1 if use_window else 0, _lib.ptr(e), edt, ld, gg.data_ptr(),
                                       None if ri is None else ri.data_ptr() + rot_col * 8,
@@ -350,7 +357,7 @@ def sc_loglik(sysmat, proj, img, rotmat=None, rotmat_inv=None, eps=0.0):
 def compton_loglik(records, row_id, coor, img, eff=None, eps=0.0):
     """Projections ``f [E]`` (in an order of its own: sorted by efficiency row) and the gradient
     ``[V, 1]`` of ``sum log(max(f, eps))`` in the image, strict model (jscc_compton_loglik); None where
-    the grid is too large for stored rows."""
+    the grid is too large for stored rows or memory too short."""
     dev = _lib.require_cuda(records, row_id, coor, img, eff, what="compton_loglik")
     c = _f32_contig(coor)
     V = c.size(0)
@@ -365,9 +372,11 @@ def compton_loglik(records, row_id, coor, img, eff=None, eps=0.0):
         return None
     if e is not None and n > 1:
         records, row_id, _ = _row_sorted_events(records, row_id)
+    ws = _lib.workspace.get(dev, nbytes, 0)
+    if ws.numel() < nbytes:
+        return None
     f = torch.empty(n, dtype=torch.float32, device=dev)
     grad = torch.zeros((V, 1), dtype=torch.float32, device=dev)
-    ws = _lib.workspace.get(dev, nbytes)
     rc = lib.jscc_compton_loglik(records.data_ptr(), row_id.data_ptr(), n, c.data_ptr(), V, _lib.ptr(e), edt, ld,
                                  x.data_ptr(), float(eps), f.data_ptr(), grad.data_ptr(), ws.data_ptr(), ws.numel(),
                                  _lib.stream_handle(dev))
@@ -631,7 +640,7 @@ def compton_weight(records, row_id, coor, img, model=_lib.CONE_STRICT, eff=None,
         # events a CTA handles share those rows in L1/L2 (only float32 rounding changes)
         records, row_id, _ = _row_sorted_events(records, row_id)
     lib = _lib.load()
-    ws = _lib.workspace.get(dev, lib.jscc_compton_weight_workspace_bytes(n, V))
+    ws = _compton_scratch(lib, dev, n, V, 0, model, use_window)
     rc = lib.jscc_compton_weight(
         records.data_ptr(), row_id.data_ptr(), n, c.data_ptr(), V, int(model), 1 if use_window else 0, _lib.ptr(e),
         edt, ld, x.data_ptr(), rm, ri, ld_rot, float(scale), out.data_ptr(), ws.data_ptr(), ws.numel(),
@@ -727,7 +736,7 @@ class ComptonBatch:
         e, edt, ld = _eff_args(eff)
         lib = _lib.load()
         for b, rec, rid in self.alone:
-            ws = _lib.workspace.get(dev, lib.jscc_compton_weight_workspace_bytes(rec.size(0), self.V))
+            ws = _compton_scratch(lib, dev, rec.size(0), self.V, 0, _lib.CONE_STRICT, False)
             rc = lib.jscc_compton_weight(
                 rec.data_ptr(), rid.data_ptr(), rec.size(0), c.data_ptr(), self.V, _lib.CONE_STRICT, 0, _lib.ptr(e),
                 edt, ld, X[b].data_ptr(), None, None, 0, float(scale), out[b].data_ptr(), ws.data_ptr(), ws.numel(),
