@@ -16,6 +16,8 @@ from . import _compton, _lib, ops
 from .compton_sparse_ops import pack_sparse_event_rows, reduce_fine_rows_to_coarse, tables
 from .process_list_plane_strict import ROW_BATCH
 
+BUILD_BLOCK_BYTES = 2 << 30  # rows of candidate events built at a time
+
 
 def _filter_unstable_event_kernels_sparse(t, t_compton, t_single):
     """Normalise the three row sets and keep effective support >= 50 (:15-22)."""
@@ -40,17 +42,24 @@ def build_sparse_rows_from_smeared(sysmat, detector, sparse_projector, list_smea
     sys_d = sysmat.to(dev)
     coor_c = sparse_projector.coor_coarse.to(dev, torch.float32)
     if vc <= _lib.SPARSE_BUILD_MAX_COARSE:
-        # one kernel writes every surviving row in place; dropped events (few: the selection has
-        # already removed the unphysical ones) cost one compaction copy
+        # one kernel writes every surviving row of a block of events in place; dropped events cost one
+        # compaction copy of the kept rows, and rows of candidates are held for one block only
         cp = sparse_projector
         if sys_d.ndim != 2 or sys_d.size(1) != cp.fine_pixel_num:
             raise ValueError("rows_fine size does not match projector.fine_pixel_num.")
+        if sys_d.dtype not in (torch.float32, torch.bfloat16):
+            sys_d = sys_d.float()  # once for all blocks
         tb = tables(cp, dev)
-        rows, keep = ops.sparse_build_rows(rec, rid, coor_c, sys_d, tb.red, tb.red_single, cp.coarse_z_num,
-                                           cp.fine_z_num, cp.coarse_layer_num, cp.fine_layer_num,
-                                           _compton.MIN_EVENT_EFFECTIVE_SUPPORT)
-        kept = torch.nonzero(keep).flatten()
-        return rows if kept.numel() == rows.size(0) else rows.index_select(0, kept)
+        block = max(1, BUILD_BLOCK_BYTES // (4 * (vc + 1)))
+        out = []
+        for a in range(0, idx.numel(), block):
+            rows, keep = ops.sparse_build_rows(rec[a:a + block], rid[a:a + block], coor_c, sys_d, tb.red,
+                                               tb.red_single, cp.coarse_z_num, cp.fine_z_num, cp.coarse_layer_num,
+                                               cp.fine_layer_num, _compton.MIN_EVENT_EFFECTIVE_SUPPORT)
+            kept = torch.nonzero(keep).flatten()
+            out.append(rows if kept.numel() == rows.size(0) else rows.index_select(0, kept))
+            del rows  # before the next block's
+        return out[0] if len(out) == 1 else torch.cat(out, dim=0)
     out = []
     for a in range(0, idx.numel(), ROW_BATCH):
         b = min(idx.numel(), a + ROW_BATCH)
