@@ -6,6 +6,7 @@ and every compute wrapper refuses non-CUDA tensors.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import threading
 from ctypes import POINTER, c_float, c_int, c_int32, c_int64, c_size_t, c_uint, c_ulonglong, c_void_p
@@ -389,18 +390,35 @@ class _Workspace:
     A CUDA graph keeps the addresses of the buffers that its kernels were captured with, so a
     buffer handed out on a stream under capture is not released when that stream's buffer grows:
     the graph may be replayed after that. Such a stream's buffers grow at least by half, so the
-    kept ones together are smaller than twice the last; ``clear`` gives all of them back."""
+    kept ones together are smaller than twice the last; ``clear`` gives all of them back. Who captures
+    a graph and holds it can have its scratch to itself instead (``owned_by``): no other graph or
+    stream works in it, and it goes when its owner goes."""
 
     def __init__(self) -> None:
         self._bufs: dict[tuple[int, int], torch.Tensor] = {}
         self._refused: dict[tuple[int, int], int] = {}
         self._captured: set[tuple[int, int]] = set()
         self._kept: list[torch.Tensor] = []
+        self._owner = threading.local()  # .buffers: of this thread's innermost owned_by
+
+    @contextlib.contextmanager
+    def owned_by(self, buffers: list):
+        """Inside, this thread's scratch comes from ``buffers`` (appended to as it has to grow; the earlier
+        ones stay, as captured kernels may use them)."""
+        outer = getattr(self._owner, "buffers", None)
+        self._owner.buffers = buffers
+        try:
+            yield buffers
+        finally:
+            self._owner.buffers = outer
 
     def get(self, device: torch.device, nbytes: int, at_least: int | None = None) -> torch.Tensor:
         """At least ``nbytes`` of scratch; where they cannot be had and the caller can work in less,
         ``at_least`` of them (a request that failed is not tried again before ``clear``: each trial
         would wait for the device and empty torch's cache)."""
+        own = getattr(self._owner, "buffers", None)
+        if own is not None:
+            return self._grow_own(own, device, nbytes, at_least)
         key = (device.index if device.index is not None else torch.cuda.current_device(),
                stream_handle(device))
         if key not in self._captured and torch.cuda.is_current_stream_capturing():
@@ -424,6 +442,17 @@ class _Workspace:
             self._kept.append(buf)
         self._bufs[key] = new
         return new
+
+    @staticmethod
+    def _grow_own(own: list, device: torch.device, nbytes: int, at_least: int | None) -> torch.Tensor:
+        if not own or own[-1].numel() < nbytes:
+            try:
+                own.append(torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device))
+            except torch.OutOfMemoryError:
+                if at_least is None or at_least >= nbytes:
+                    raise
+                return _Workspace._grow_own(own, device, at_least, None)
+        return own[-1]
 
     def clear(self) -> None:
         self._bufs.clear()

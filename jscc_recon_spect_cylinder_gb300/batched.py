@@ -95,6 +95,7 @@ class BatchedScOsem:
         self.W = torch.empty((V, self.nr), dtype=torch.float32, device=dev)
         self.splits = {}
         self.graph = None
+        self._scratch = []  # what the graph's kernels work in
         self.graph_launches = 0
         self.floor = None  # clamp_min of the forward projection (joint local loops: 1e-12)
 
@@ -194,11 +195,12 @@ class BatchedScOsem:
         torch.cuda.synchronize(self.dev)
         self.X.copy_(saved)
         g = torch.cuda.CUDAGraph()
+        scratch = []  # the graph's own: replays of other objects' graphs do not share it
         n0 = _lib.launch_count()
-        with torch.cuda.graph(g):
+        with torch.cuda.graph(g), _lib.workspace.owned_by(scratch):
             self._iteration()
         self.graph_launches = _lib.launch_count() - n0  # kernels one replay launches
-        self.graph = g
+        self.graph, self._scratch = g, scratch
         return g
 
 
