@@ -249,16 +249,19 @@ FP32_PEAK_SOURCE = ("nominal: 152 SMs x 128 FP32 lanes x 2 FLOP per FMA x 2.07 G
 
 def cone_flop_per_pair(kernels):
     """FP32 FLOPs per fully evaluated event-voxel pair of the strict cone ``kernels`` (their
-    average), from ncu's FP32 instruction counters (profiles/cone_flops_jsccd2.json: FADD,
-    FMUL = 1, FFMA, FADD2, FMUL2 = 2, FFMA2 = 4 per thread instruction, over the launch's
-    event-voxel pairs; the special-function unit's instructions, compares and selects are not
-    counted); the formula's hand count (Cone2Bench.K_CONE) when no capture is committed."""
+    average; a dict gives the pairs that each evaluates), from ncu's FP32 instruction counters
+    (profiles/cone_flops_jsccd2.json: FADD, FMUL = 1, FFMA, FADD2, FMUL2 = 2, FFMA2 = 4 per
+    thread instruction, over the launch's event-voxel pairs; the special-function unit's
+    instructions, compares and selects are not counted); the formula's hand count
+    (Cone2Bench.K_CONE) when no capture is committed."""
     f = REPO / "profiles" / "cone_flops_jsccd2.json"
     if f.exists():
         d = json.loads(f.read_text())
-        vals = [d[k]["flop_per_pair"] for k in kernels if k in d]
-        if vals:
-            return float(np.mean(vals)), "ncu FP32 instruction counters (profiles/cone_flops_jsccd2.json)"
+        known = [k for k in kernels if k in d]
+        pairs = [kernels[k] if isinstance(kernels, dict) else 1.0 for k in known]
+        if sum(pairs) > 0:
+            fpp = np.average([d[k]["flop_per_pair"] for k in known], weights=pairs)
+            return float(fpp), "ncu FP32 instruction counters (profiles/cone_flops_jsccd2.json)"
     return float(Cone2Bench.K_CONE), "hand count of the strict formula"
 
 
@@ -496,19 +499,14 @@ class Map5Bench:
                 "l2": "SC matrix 11.8 GB > L2 (read once per step); records 90 MB"}
 
     def extra(self, ms_per_step):
-        """The FP32 roofline of the step's cone passes (forward + adjoint over every pair),
-        timed on their own."""
+        """The FP32 roofline of the step's cone pass (projections and gradient, every pair
+        evaluated once), timed on its own."""
         from jscc_recon_spect_cylinder_gb300 import ops
 
         x = torch.ones((self.V, 1), device=self.dev)
-        g = torch.ones(len(self.ev), device=self.dev)
 
         def cone_pass():
-            f = ops.compton_project(self.ev.records, self.ev.row_id, self.coor, x, model=self.ev.model, eff=self.eff,
-                                    use_window=False)
-            ops.compton_backproject(self.ev.records, self.ev.row_id, self.coor, g, model=self.ev.model, eff=self.eff,
-                                    use_window=False)
-            return f
+            return ops.compton_loglik(self.ev.records, self.ev.row_id, self.coor, x, eff=self.eff)
 
         cone_pass()
         torch.cuda.synchronize(self.dev)
@@ -518,9 +516,10 @@ class Map5Bench:
         t1.record()
         torch.cuda.synchronize(self.dev)
         ms = t0.elapsed_time(t1)
-        pairs = 2 * len(self.ev) * self.V
+        pairs = len(self.ev) * self.V
         return {"cone_pass": {"pairs_per_s": pairs / (ms / 1e3), "ms": ms},
-                "fp32_roofline": cone_roofline(pairs / (ms / 1e3))}
+                "fp32_roofline": cone_roofline(pairs / (ms / 1e3), over="the step's cone pass",
+                                               kernels=("cone_rows_pair",))}
 
 
 class Batch4Bench:
@@ -848,7 +847,7 @@ class Batch4JointBench(Batch4Bench):
 
     def extra(self, ms_per_step):
         """Cone pairs per second over the whole step (the cone kernels take nearly all of it),
-        the FP32 roofline at Cone2Bench's operations per pair, the plain FP32 single-instance
+        the FP32 roofline at the operations per pair of the kernels that evaluate them, the plain FP32 single-instance
         joint path run for the 64 instances in turn, and per-instance errors against float64."""
         pairs = 2 * self.n_kept * self.V  # forward + back cone pairs per iteration
         # instances weighted by themselves evaluate each pair once, the batch's twice
@@ -857,7 +856,10 @@ class Batch4JointBench(Batch4Bench):
         value = self.units_per_step() / (ms_per_step / 1e3)
         seq = self._sequential_fp32()
         return {"compton_pairs_per_s": rate,
-                "fp32_roofline": cone_roofline((pairs - alone) / (ms_per_step / 1e3), over="the whole step"),
+                "fp32_roofline": cone_roofline(
+                    (pairs - alone) / (ms_per_step / 1e3), over="the whole step",
+                    kernels={"cone_forward_pair": pairs / 2 - alone, "cone_back_pair": pairs / 2 - alone,
+                             "cone_rows_pair": alone}),
                 "sequential_fp32_joint_64_instances": {"subset_iters_per_s": seq,
                                                        "batched_speedup_vs_64_sequential": value / seq},
                 "errors_vs_fp64": self._errors()}
