@@ -455,7 +455,7 @@ cone_forward_kernel(const ConeEvent* __restrict__ rec, const int32_t* __restrict
   if (tid < EB) {
     const int64_t i = i0 + tid < n_ev ? i0 + tid : n_ev - 1;
     sev[tid] = Stage::stage(rec[i]);
-    srow[tid] = (int64_t)row_id[i] * ld_eff;
+    srow[tid] = eff ? (int64_t)row_id[i] * ld_eff : 0;
   }
   __syncthreads();
   const int ne = (n_ev - i0) < EB ? (int)(n_ev - i0) : EB;
@@ -598,7 +598,7 @@ cone_back_kernel(const ConeEvent* __restrict__ rec, const int32_t* __restrict__ 
     __syncthreads();
     if (tid < n) {
       sev[tid] = Stage::stage(rec[s + tid]);
-      srow[tid] = (int64_t)row_id[s + tid] * ld_eff;
+      srow[tid] = eff ? (int64_t)row_id[s + tid] * ld_eff : 0;
       sq[tid] = q[s + tid];
     }
     __syncthreads();
@@ -780,7 +780,7 @@ cone_forward_pair_kernel(const ConeEvent* __restrict__ rec, const int32_t* __res
   if (tid < EB) {
     const int64_t i = i0 + tid < n_ev ? i0 + tid : n_ev - 1;  // padding repeats a valid event
     stage_pair_half(&sev[tid >> 1], tid & 1, rec[i]);
-    srow[tid] = (int64_t)row_id[i] * ld_eff;
+    srow[tid] = eff ? (int64_t)row_id[i] * ld_eff : 0;
   }
   __syncthreads();
   const int ne = (n_ev - i0) < EB ? (int)(n_ev - i0) : EB;
@@ -865,12 +865,12 @@ cone_back_pair_kernel(const ConeEvent* __restrict__ rec, const int32_t* __restri
     __syncthreads();
     if (tid < n) {
       stage_pair_half(&sev[tid >> 1], tid & 1, rec[s + tid]);
-      srow[tid] = (int64_t)row_id[s + tid] * ld_eff;
+      srow[tid] = eff ? (int64_t)row_id[s + tid] * ld_eff : 0;
       sq[tid] = q[s + tid];
     } else if (tid == n && (n & 1)) {
       // odd count: the pair's second half repeats event s with a zero ratio
       stage_pair_half(&sev[tid >> 1], 1, rec[s]);
-      srow[tid] = (int64_t)row_id[s] * ld_eff;
+      srow[tid] = eff ? (int64_t)row_id[s] * ld_eff : 0;
       sq[tid] = 0.f;
     }
     __syncthreads();
@@ -927,7 +927,7 @@ cone_rows_pair_kernel(const ConeEvent* __restrict__ rec, const int32_t* __restri
   if (tid < kRowsStage) {
     const int64_t i = i0 + (tid < n ? tid : n - 1);  // an odd count's second half repeats its event
     stage_pair_half(&sev[tid >> 1], tid & 1, rec[i]);
-    srow[tid] = (int64_t)row_id[i] * ld_eff;
+    srow[tid] = eff ? (int64_t)row_id[i] * ld_eff : 0;
   }
   __syncthreads();
   if (j >= V) return;
