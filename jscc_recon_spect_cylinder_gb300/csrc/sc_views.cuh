@@ -9,7 +9,7 @@
 //                     TM * NB FMAs on TM loads of A and NB / 4 16-byte reads of x. One transposing
 //                     butterfly per row group; partial sums per slice
 //   sc_views_ratio    q[b][r] = y[b, r] / f, slices in order (or f itself)
-//   sc_views_back     CTA = 128 columns x a chunk of rows; a lane holds 4 NB sums, a row's NB ratios
+//   sc_views_back     CTA = 128 (or 256) columns x a chunk of rows; a lane holds 4 NB (8 NB) sums, a row's NB ratios
 //                     are one broadcast; the eight warps take every eighth row and add up in warp order
 // then sc_reduce_scatter_kernel (views and chunks in order).
 // Bound: HBM below about 8 views, the FP32 pipe (2 NB flops an element and pass at 80 TFLOP/s) and
@@ -42,14 +42,20 @@ struct SvTraits {
   static constexpr int kFwdRing = RING ? kSvWarps * kFwdStages * kRows * 128 : 0;  // bytes of a CTA
 };
 
+// Columns of a back pass's tile. Aligned BF16 rows of few views: 256, so that a warp reads 512 bytes of a
+// row, as it does of float32: 256 bytes at a time ran at 2.6 to 3.8 TB/s, 512 at 5.1 to 5.4 (back projection
+// of two views, 41,666 x 4,800: 153 -> 75 us, 5,555 x 36,000: 126 -> 79 us). The sums of more views leave no
+// registers for that.
+constexpr int sv_back_cols(int nb, size_t el, bool aligned) { return aligned && el == 2 && nb <= 4 ? 256 : 128; }
+
 // The back pass's copies. COPY 0: plain loads, a row ahead; 1: four-byte cp.async units; 2: a lane's
-// four columns in one cp.async (16 bytes of float32, 8 of BF16), for rows on such boundaries.
+// columns in one cp.async of 16 bytes (8 for BF16 of more views), for rows on such boundaries.
 template <typename T, int NB, int COPY>
 struct SvBack {
-  static constexpr int kCols = 4;  // columns of a lane
+  static constexpr int kCols = sv_back_cols(NB, sizeof(T), COPY == 2) / 32;  // columns of a lane
   static constexpr int kUnit = COPY == 2 ? kCols : COPY == 1 ? 4 / (int)sizeof(T) : 1;  // columns of a copy
   static constexpr int kUnits = kCols / kUnit;
-  static constexpr int kStages = sizeof(T) == 2 ? 16 : 8;
+  static constexpr int kStages = 32 * kCols * sizeof(T) == 256 ? 16 : 8;
   // a row's ratios (in whole 16 bytes), then its units
   static constexpr int kRatioBytes = (NB * 4 + 15) / 16 * 16;
   static constexpr int kStage = 32 * kCols * (int)sizeof(T) + kRatioBytes;
@@ -57,7 +63,6 @@ struct SvBack {
   static constexpr int kSum = kSvWarps * NB * 32 * kCols * 4;
   static constexpr int kSmem = kRing > kSum ? kRing : kSum;
 };
-constexpr int kSvBackCols = 128;
 
 // the columns of a unit as floats
 template <typename T, int UNIT>
@@ -94,6 +99,7 @@ inline int sv_pad(int views) {
 inline int sv_pitch(int nb) { return nb == 2 ? 2 : ((nb / 4) % 2 ? nb : nb + 4); }
 inline int sv_rows(int nb) { return nb == 2 ? 16 : 8; }
 inline int sv_fwd_ctas(int nb) { return nb <= 8 ? 2 : 1; }
+constexpr int sv_back_ctas(int nb) { return nb <= 4 ? 3 : nb <= 12 ? 2 : 1; }
 inline size_t sv_fwd_ring(int nb) { return (size_t)kSvWarps * (nb <= 8 ? 4 : 8) * sv_rows(nb) * 128; }
 
 // xt[j * pitch + r] = img[rotmat[j, r0 + r] - 1] (the image itself without a table), 0 for r >= nr
@@ -339,15 +345,16 @@ sc_views_ratio_kernel(const float* __restrict__ part, int n_slices, int64_t n_bi
 
 // part[(chunk * NB + r) * ldp + j] = sum over the chunk's rows b of A[row(b), j] ratio[b * NB + r]
 template <typename T, int NB, int COPY>
-__global__ void __launch_bounds__(kSvThreads, NB <= 4 ? 3 : NB <= 12 ? 2 : 1)
+__global__ void __launch_bounds__(kSvThreads, sv_back_ctas(NB))
 sc_views_back_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __restrict__ row_idx, int64_t n_bins,
                      int64_t V, const float* __restrict__ ratio, int64_t rows_per_chunk, float* __restrict__ part,
                      int64_t ldp) {
   using Tr = SvBack<T, NB, COPY>;
+  constexpr int COLS = 32 * Tr::kCols;
   constexpr int TC = Tr::kCols, NP = NB / 2, E = Tr::kUnit, TU = Tr::kUnits, D = Tr::kStages;
   extern __shared__ __align__(128) unsigned char sv_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t c0 = (int64_t)blockIdx.x * kSvBackCols;
+  const int64_t c0 = (int64_t)blockIdx.x * COLS;
   const int64_t b_begin = (int64_t)blockIdx.y * rows_per_chunk;
   const int64_t b_end = b_begin + rows_per_chunk < n_bins ? b_begin + rows_per_chunk : n_bins;
   // the lane's column t * E + e stands at (32 t + lane) E + e of the tile
@@ -383,7 +390,7 @@ sc_views_back_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __rest
     }
   };
   // a tile whose last columns fill no whole unit takes the plain loads
-  const bool whole = E == 1 || V - c0 >= kSvBackCols || (V - c0) % E == 0;
+  const bool whole = E == 1 || V - c0 >= COLS || (V - c0) % E == 0;
   if (COPY != 0 && whole) {
     int64_t col[TU];  // units past the matrix repeat its last one (their sums are not written)
 #pragma unroll
@@ -422,6 +429,10 @@ sc_views_back_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __rest
       if constexpr (COPY == 2 && sizeof(T) == 4) {
         const float4 v = *reinterpret_cast<const float4*>(st + lane * 16);
         a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
+      } else if constexpr (COPY == 2 && TC == 8) {
+        const uint4 v = *reinterpret_cast<const uint4*>(st + lane * 16);
+        a[0] = bf16_lo(v.x); a[1] = bf16_hi(v.x); a[2] = bf16_lo(v.y); a[3] = bf16_hi(v.y);
+        a[4] = bf16_lo(v.z); a[5] = bf16_hi(v.z); a[6] = bf16_lo(v.w); a[7] = bf16_hi(v.w);
       } else if constexpr (COPY == 2) {
         const uint2 v = *reinterpret_cast<const uint2*>(st + lane * 8);
         a[0] = bf16_lo(v.x); a[1] = bf16_hi(v.x); a[2] = bf16_lo(v.y); a[3] = bf16_hi(v.y);
@@ -438,7 +449,7 @@ sc_views_back_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __rest
     }
     cp_async_wait<0>();
   } else {
-    constexpr int U = 4;  // rows loaded together
+    constexpr int U = TC == 8 ? 1 : 4;  // rows loaded together
     int64_t cs[TC];
 #pragma unroll
     for (int t = 0; t < TC; ++t) cs[t] = c0 + column(t) < V ? c0 + column(t) : V - 1;
@@ -470,7 +481,7 @@ sc_views_back_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __rest
     }
   }
   __syncthreads();  // the rings are free
-  float(*red)[NB][kSvBackCols] = reinterpret_cast<float(*)[NB][kSvBackCols]>(sv_smem);
+  float(*red)[NB][COLS] = reinterpret_cast<float(*)[NB][COLS]>(sv_smem);
 #pragma unroll
   for (int t = 0; t < TC; ++t)
 #pragma unroll
@@ -479,8 +490,8 @@ sc_views_back_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __rest
       red[warp][2 * k + 1][column(t)] = acc[t][k].y;
     }
   __syncthreads();
-  for (int i = tid; i < NB * kSvBackCols; i += kSvThreads) {
-    const int r = i / kSvBackCols, c = i % kSvBackCols;
+  for (int i = tid; i < NB * COLS; i += kSvThreads) {
+    const int r = i / COLS, c = i % COLS;
     if (c0 + c >= V) continue;
     float sum = red[0][r][c];
 #pragma unroll
@@ -506,7 +517,7 @@ static size_t sv_bytes(const SvPlan& p, int64_t n_bins, int64_t V) {
   return b + 256;
 }
 
-static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap) {
+static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap, size_t el) {
   const int64_t sms = num_sms();
   SvPlan p{};
   p.ldp = (int64_t)align_up((size_t)V, 8);
@@ -518,7 +529,7 @@ static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap) {
     const int64_t units = (V + 63) / 64;
     const int64_t group = (int64_t)kSvWarps * sv_rows(p.nb);
     const int64_t groups = (n_bins + group - 1) / group;
-    // forward: the fewest slices that fit shared memory whole, more while row groups leave SMs idle
+    // forward: at least the slices that fit shared memory whole, more while row groups leave SMs idle
     const int64_t wave = sms * sv_fwd_ctas(p.nb);
     const int64_t cols_fit =
         (int64_t)((kSvSmem / sv_fwd_ctas(p.nb) - sv_fwd_ring(p.nb)) / (p.pitch * sizeof(float))) / 64 * 64;
@@ -527,9 +538,41 @@ static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap) {
     if (slices < want) slices = want;
     if (slices > units) slices = units;
     // back: about two CTAs an SM, at least eight rows a warp
-    const int64_t tiles = (V + kSvBackCols - 1) / kSvBackCols;
+    const int64_t tile = sv_back_cols(p.nb, el, true), tiles = (V + tile - 1) / tile;
+    const int64_t most = (n_bins + 63) / 64;
     int64_t chunks = (2 * sms + tiles - 1) / tiles;
-    if (chunks > (n_bins + 63) / 64) chunks = (n_bins + 63) / 64;
+    if (chunks > most) chunks = most;
+    // Then a few more of either where they fill the rounds of CTAs better: the passes' bytes over the share of
+    // the CTA slots that work, a round's start and end (about 1 us + 0.1 us a view at 6.5 TB/s) and the partial
+    // sums written and read. Two views: projection of 20,833 float32 rows of 4,800 voxels 146 -> 89 us (one
+    // slice: 163 CTAs on 304 slots; nine: five rounds, 97% of them at work), weight of 2,777 x 36,000 164 -> 158.
+    const double work = (double)n_bins * (double)V * (double)el, turn = 0.65e6 * (double)(10 + p.nb);
+    auto cheapest = [](int64_t first, int64_t last, auto cost) {
+      int64_t best = first;
+      double least = cost(first);
+      for (int64_t k = first + 1; k <= last; ++k) {
+        const double c = cost(k);
+        if (c < least) {
+          least = c;
+          best = k;
+        }
+      }
+      return best;
+    };
+    slices = cheapest(slices, slices + 8 < units ? slices + 8 : units, [&](int64_t k) {
+      const int64_t splits = wave / k < 1 ? 1 : (wave / k < groups ? wave / k : groups);
+      const double rounds = (double)((groups + splits - 1) / splits) * (double)((k * splits + wave - 1) / wave);
+      return work * rounds * (double)wave / (double)(groups * k) + turn * rounds +
+             8.0 * (double)(k * n_bins * p.nb);
+    });
+    const int64_t slots = sms * sv_back_ctas(p.nb);
+    chunks = cheapest(chunks, chunks + 8 < most ? chunks + 8 : most, [&](int64_t k) {
+      // (two CTAs of three already draw the full rate: a last round of fewer takes as long as theirs)
+      const int64_t full = tiles * k / slots, rest = tiles * k % slots, least = 2 * slots / 3;
+      const double share = (double)(full * slots + (rest == 0 ? 0 : rest < least ? least : rest));
+      return work * share / (double)(tiles * k) + turn * (double)(full + (rest > 0)) +
+             8.0 * (double)(k * p.nb) * (double)V;
+    });
     for (;;) {
       p.slices = (int)slices;
       p.rows_per_chunk = (n_bins + chunks - 1) / chunks;
@@ -569,23 +612,24 @@ static int sv_launch_block(const T* A, int64_t lda, const int64_t* row_idx, int6
     JSCC_LAUNCH_CHECK();
     if (stage == 1) return JSCC_OK;
   }
-  const int64_t tiles = (V + kSvBackCols - 1) / kSvBackCols;
-  auto back = [&](auto kernel, int smem) {
+  auto back = [&](auto kernel, int smem, int cols) {
     cudaError_t e = allow_smem(kernel);
     if (e != cudaSuccess) return e;
     JSCC_TIMED("sc_views_back", st,
-               (kernel<<<dim3((unsigned)tiles, (unsigned)p.chunks), kSvThreads, smem, st>>>(
+               (kernel<<<dim3((unsigned)((V + cols - 1) / cols), (unsigned)p.chunks), kSvThreads, smem, st>>>(
                    A, lda, row_idx, n_bins, V, ratio, p.rows_per_chunk, part, p.ldp)));
     return cudaSuccess;
   };
-  const int quad = 4 * (int)sizeof(T);
-  const bool quads = (lda * (int64_t)sizeof(T)) % quad == 0 && reinterpret_cast<uintptr_t>(A) % quad == 0;
+  using Wide = SvBack<T, NB, 2>;
+  const int unit = Wide::kUnit * (int)sizeof(T);
+  const bool whole = (lda * (int64_t)sizeof(T)) % unit == 0 && reinterpret_cast<uintptr_t>(A) % unit == 0;
   // rows on odd boundaries: four-byte copies pay from 12 views on, where the plain loads' registers
   // leave one CTA an SM (2,048 x 35,343 float32, 8 views: plain 68 us, copies 125 us; 512 rows, 20
   // views: copies 51 us)
   constexpr int kOdd = (RING && NB >= 12) ? 1 : 0;
-  JSCC_CUDA_CHECK(quads ? back(sc_views_back_kernel<T, NB, 2>, SvBack<T, NB, 2>::kSmem)
-                        : back(sc_views_back_kernel<T, NB, kOdd>, SvBack<T, NB, kOdd>::kSmem));
+  JSCC_CUDA_CHECK(whole ? back(sc_views_back_kernel<T, NB, 2>, Wide::kSmem, 32 * Wide::kCols)
+                        : back(sc_views_back_kernel<T, NB, kOdd>, SvBack<T, NB, kOdd>::kSmem,
+                               32 * SvBack<T, NB, kOdd>::kCols));
   JSCC_LAUNCH_CHECK();
   return JSCC_OK;
 }
@@ -598,7 +642,7 @@ static int sc_views(const T* A, int64_t lda, const int64_t* row_idx, int64_t n_b
                     int64_t ld_rot, int mode, float floor_v, int has_scale, float scale, float* weight,
                     void* ws, size_t ws_bytes, cudaStream_t st, int stage, float* fout, int64_t ld_fout,
                     const float* gin, int64_t ld_gin) {
-  const SvPlan p = plan_views(n_bins, V, n_rot, ws_bytes);
+  const SvPlan p = plan_views(n_bins, V, n_rot, ws_bytes, sizeof(T));
   JSCC_REQUIRE(p.bytes <= ws_bytes, "SC projector: %d views need %zu bytes of workspace (%zu given)", n_rot, p.bytes,
                ws_bytes);
   Carver cv(ws, ws_bytes);
