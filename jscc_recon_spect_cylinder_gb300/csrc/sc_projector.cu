@@ -127,8 +127,9 @@ __device__ __forceinline__ float fma_raw<__nv_bfloat16>(const uint4& u, const fl
 // fewer), so all warps stream the same number of bytes. A range crosses at most a
 // few row boundaries; for each row piece the warp writes one partial dot product
 // to part[g][k]. sc_finish_ratio_kernel sums a row's partials in warp order. The image is staged
-// in shared memory when it fits.
-template <typename T, bool VEC, bool SMEM_X, int THREADS>
+// in shared memory when it fits. VIEWS = 2: two images, x[j][2], with two partials a piece (staged one after
+// the other, xs[r][ldx]).
+template <typename T, bool VEC, bool SMEM_X, int THREADS, int VIEWS = 1>
 __global__ void __launch_bounds__(THREADS)
 sc_forward_split_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __restrict__ row_idx,
                         int64_t n_bins, int64_t V, const float* __restrict__ x, int64_t nvr, int64_t L, int maxp,
@@ -139,8 +140,12 @@ sc_forward_split_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __r
   float* xs = reinterpret_cast<float*>(xs4);
   const int lane = threadIdx.x & 31;
   const int64_t g = (int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
+  static_assert(VIEWS == 1 || SMEM_X, "two images are staged");
+  const int ldx = VIEWS == 1 ? 0 : (int)((V + 7) / 8 * 8);
   if (SMEM_X) {
-    for (int64_t i = threadIdx.x; i < V; i += THREADS) xs[i] = __ldg(x + i);
+    for (int64_t i = threadIdx.x; i < V; i += THREADS)
+#pragma unroll
+      for (int r = 0; r < VIEWS; ++r) xs[r * ldx + i] = __ldg(x + i * VIEWS + r);
     __syncthreads();
   }
   const float* xsrc = SMEM_X ? xs : x;
@@ -154,7 +159,9 @@ sc_forward_split_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __r
     const int64_t piece_end = row_end < u_end ? row_end : u_end;
     const T* rowp = A + (row_idx ? row_idx[row] : row) * lda;
     const int64_t ubase = row * nvr;
-    float acc = 0.f;
+    float acc[VIEWS];
+#pragma unroll
+    for (int r = 0; r < VIEWS; ++r) acc[r] = 0.f;
     int64_t uu = u + lane;
     if constexpr (VEC) {
       // 4 independent 16-byte loads in flight per lane; raw registers, converted on use.
@@ -173,7 +180,8 @@ sc_forward_split_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __r
           for (int q = 0; q < 4; ++q) raw[q] = ld_stream_u4(rp + col + 32 * NV * q);
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            acc = fma_raw<T>(raw[q], xp0 + col + 32 * NV * q, acc);
+#pragma unroll
+            for (int r = 0; r < VIEWS; ++r) acc[r] = fma_raw<T>(raw[q], xp0 + r * ldx + col + 32 * NV * q, acc[r]);
         }
         uu += (int64_t)n_iter * 128;
       }
@@ -186,53 +194,71 @@ sc_forward_split_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __r
           float a[NV];
           load_vec<T>(rowp + col, a);
 #pragma unroll
-          for (int kk = 0; kk < NV; ++kk) acc = fmaf(a[kk], xsrc[col + kk], acc);
+          for (int r = 0; r < VIEWS; ++r)
+#pragma unroll
+            for (int kk = 0; kk < NV; ++kk) acc[r] = fmaf(a[kk], xsrc[r * ldx + col + kk], acc[r]);
           done = true;
         }
       }
       if (!done) {
         const int64_t cend = (col + NV < V) ? col + NV : V;
-        for (int64_t c = col; c < cend; ++c) acc = fmaf(load_elem(rowp, c), xsrc[c], acc);
+        for (int64_t c = col; c < cend; ++c) {
+          const float a = load_elem(rowp, c);
+#pragma unroll
+          for (int r = 0; r < VIEWS; ++r) acc[r] = fmaf(a, xsrc[r * ldx + c], acc[r]);
+        }
       }
     }
-    const float sum = warp_sum(acc);
-    if (lane == 0) part[g * maxp + k] = sum;
+#pragma unroll
+    for (int r = 0; r < VIEWS; ++r) {
+      const float sum = warp_sum(acc[r]);
+      if (lane == 0) part[(g * maxp + k) * VIEWS + r] = sum;
+    }
     ++k;
     ++row;
     u = piece_end;
   }
 }
 
-// f of row b: the row's partials in warp order
-__device__ __forceinline__ float row_sum(const float* __restrict__ part, int64_t b, int64_t nvr, int64_t L, int maxp) {
+// f of row b (in view r): the row's partials in warp order
+template <int VIEWS>
+__device__ __forceinline__ float row_sum(const float* __restrict__ part, int64_t b, int r, int64_t nvr, int64_t L,
+                                         int maxp) {
   const int64_t g0 = (b * nvr) / L;
   const int64_t g1 = ((b + 1) * nvr - 1) / L;
   float f = 0.f;
   for (int64_t g = g0; g <= g1; ++g) {
     const int64_t first_row = (g * L) / nvr;
-    f += part[(g * maxp) + (b - first_row)];
+    f += part[((g * maxp) + (b - first_row)) * VIEWS + r];
   }
   return f;
 }
 
-// ratio[b] = row_ratio(proj[b], f), and f_out[b] = f where it is given
+// ratio[b] = row_ratio(proj[b], f), and f_out[b] = f where it is given (of two views: [b][2], columns 0 and 1
+// of proj and f_out)
+template <int VIEWS>
 __global__ void sc_finish_ratio_kernel(const float* __restrict__ part, int64_t n_bins, int64_t nvr,
                                        int64_t L, int maxp, const int64_t* __restrict__ row_idx,
                                        const float* __restrict__ proj, int64_t ld_proj, int mode, float floor_v,
                                        float* __restrict__ ratio, float* __restrict__ f_out, int64_t ld_f) {
-  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < n_bins; b += (int64_t)gridDim.x * blockDim.x) {
-    const float f = row_sum(part, b, nvr, L, maxp);
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n_bins * VIEWS;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = t / VIEWS;
+    const int r = (int)(t % VIEWS);
+    const float f = row_sum<VIEWS>(part, b, r, nvr, L, maxp);
     const int64_t pb = row_idx ? row_idx[b] : b;
-    if (f_out != nullptr) f_out[b * ld_f] = f;
-    ratio[b] = row_ratio(proj[pb * ld_proj], f, mode, floor_v);
+    if (f_out != nullptr) f_out[b * ld_f + r] = f;
+    ratio[t] = row_ratio(proj[pb * ld_proj + r], f, mode, floor_v);
   }
 }
 
-// out[b][r0] = f(b) (the forward projection itself, no ratio)
+// out[b][r] = f(b, r) (the forward projection itself, no ratio)
+template <int VIEWS>
 __global__ void sc_finish_raw_kernel(const float* __restrict__ part, int64_t n_bins, int64_t nvr, int64_t L,
-                                     int maxp, int r0, float* __restrict__ out, int64_t ld_out) {
-  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < n_bins; b += (int64_t)gridDim.x * blockDim.x)
-    out[b * ld_out + r0] = row_sum(part, b, nvr, L, maxp);
+                                     int maxp, float* __restrict__ out, int64_t ld_out) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n_bins * VIEWS;
+       t += (int64_t)gridDim.x * blockDim.x)
+    out[t / VIEWS * ld_out + t % VIEWS] = row_sum<VIEWS>(part, t / VIEWS, (int)(t % VIEWS), nvr, L, maxp);
 }
 
 // ratio[b * nb + r] = g[b][r0 + r] (a caller-given vector to back-project), 0 for r >= nr
@@ -623,15 +649,14 @@ static int sc_one_view(const T* A, int64_t lda, const int64_t* row_idx, int64_t 
     JSCC_LAUNCH_CHECK();
     if (stage == 1) {
       JSCC_TIMED("sc_finish_raw", st,
-                 (sc_finish_raw_kernel<<<(unsigned)row_blocks, 256, 0, st>>>(fpart, n_bins, nvr, L, p.fwd_maxp, 0,
-                                                                             fout, ld_fout)));
+                 (sc_finish_raw_kernel<1><<<(unsigned)row_blocks, 256, 0, st>>>(fpart, n_bins, nvr, L, p.fwd_maxp, fout,
+                                                                                ld_fout)));
       JSCC_LAUNCH_CHECK();
       return JSCC_OK;
     }
     JSCC_TIMED("sc_finish_ratio", st,
-               (sc_finish_ratio_kernel<<<(unsigned)row_blocks, 256, 0, st>>>(fpart, n_bins, nvr, L, p.fwd_maxp,
-                                                                             row_idx, proj, ld_proj, mode, floor_v,
-                                                                             ratio, fout, ld_fout)));
+               (sc_finish_ratio_kernel<1><<<(unsigned)row_blocks, 256, 0, st>>>(
+                   fpart, n_bins, nvr, L, p.fwd_maxp, row_idx, proj, ld_proj, mode, floor_v, ratio, fout, ld_fout)));
     JSCC_LAUNCH_CHECK();
   }
   const dim3 grid((unsigned)p.col_tiles, (unsigned)p.chunks);

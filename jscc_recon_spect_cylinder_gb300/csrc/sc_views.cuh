@@ -506,13 +506,28 @@ struct SvPlan {
   int blocks, per, nb, pitch;  // views: blocks of `per` (padded to nb)
   int slices, piece_cols, row_splits;
   int64_t chunks, rows_per_chunk, ldp;
+  int64_t ranges;  // warps of the one-view forward kernel, where two views may take it (0: they do not)
+  int maxp;        // and its row pieces a warp
   size_t bytes;
 };
+
+// Two views of float32 rows on 16-byte boundaries take the one-view forward kernel with both images in
+// shared memory where they fit and the matrix is past 96 MB: it reads whole stretches of rows, 5.6 TB/s
+// (projection of 20,833 x 4,800: 71 against 89 us, 6,944 x 14,400 71 and 88), the kernel of several views 128
+// bytes of 16 rows at a time. From L2 that is the faster (1,666 x 4,800: 12.0 against 13.4 us), as it
+// is for BF16, of three views on, and past 25,600 voxels (2,777 x 36,000: 87 against 95 us).
+constexpr int64_t kSvSplitBytes = 96000000;
+constexpr size_t kSvSplitSmem = 200 * 1024;
+
+static size_t sv_forward_floats(const SvPlan& p, int64_t n_bins) {
+  const size_t views = (size_t)p.slices * n_bins * p.nb, split = (size_t)p.ranges * p.maxp * 2;
+  return views > split ? views : split;
+}
 
 static size_t sv_bytes(const SvPlan& p, int64_t n_bins, int64_t V) {
   size_t b = align_up((size_t)V * p.pitch * sizeof(float), 256);
   b += align_up((size_t)n_bins * p.nb * sizeof(float), 256);                      // ratios
-  b += align_up((size_t)p.slices * n_bins * p.nb * sizeof(float), 256);           // forward partials
+  b += align_up(sv_forward_floats(p, n_bins) * sizeof(float), 256);               // forward partials
   b += align_up((size_t)p.chunks * p.nb * (size_t)p.ldp * sizeof(float), 256);    // back partials
   return b + 256;
 }
@@ -521,6 +536,11 @@ static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap, size_
   const int64_t sms = num_sms();
   SvPlan p{};
   p.ldp = (int64_t)align_up((size_t)V, 8);
+  if (n_rot == 2 && el == sizeof(float) && (size_t)p.ldp * 2 * sizeof(float) <= kSvSplitSmem &&
+      n_bins * V * (int64_t)el >= kSvSplitBytes) {
+    p.ranges = sms * 32;
+    p.maxp = (int)((n_bins + p.ranges - 1) / p.ranges) + 2;
+  }
   for (int blocks = (n_rot + kSvMaxViews - 1) / kSvMaxViews;; ++blocks) {
     p.blocks = blocks;
     p.per = (n_rot + blocks - 1) / blocks;
@@ -578,6 +598,10 @@ static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap, size_
       p.rows_per_chunk = (n_bins + chunks - 1) / chunks;
       p.chunks = (n_bins + p.rows_per_chunk - 1) / p.rows_per_chunk;
       p.bytes = sv_bytes(p, n_bins, V);
+      if (p.bytes > cap && p.ranges > 0) {
+        p.ranges = 0;
+        continue;
+      }
       if (p.bytes <= cap || (slices == 1 && chunks == 1)) break;
       if (slices > 1) slices = (slices + 1) / 2;
       else chunks = (chunks + 1) / 2;
@@ -597,7 +621,28 @@ static int sv_launch_block(const T* A, int64_t lda, const int64_t* row_idx, int6
                            const float* proj, int64_t ld_proj, int mode, float floor_v, int stage, float* fout,
                            int64_t ld_fout, cudaStream_t st) {
   using Tr = SvTraits<T, NB, RING>;
-  if (stage != 2) {
+  const bool split = NB == 2 && sizeof(T) == 4 && p.ranges > 0 && lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
+  if (stage != 2 && split) {
+    if constexpr (NB == 2 && sizeof(T) == 4) {
+      const int64_t nvr = (V + 3) / 4, L = (n_bins * nvr + p.ranges - 1) / p.ranges;
+      auto kernel = sc_forward_split_kernel<T, true, true, 1024, 2>;
+      JSCC_CUDA_CHECK(allow_smem(kernel));
+      JSCC_TIMED("sc_forward_split", st,
+                 (kernel<<<(unsigned)(p.ranges / 32), 1024, (size_t)p.ldp * 2 * sizeof(float), st>>>(
+                     A, lda, row_idx, n_bins, V, xt, nvr, L, p.maxp, fpart)));
+      JSCC_LAUNCH_CHECK();
+      const unsigned blocks = (unsigned)((2 * n_bins + 255) / 256);
+      if (stage == 1)
+        JSCC_TIMED("sc_finish_raw", st,
+                   (sc_finish_raw_kernel<2><<<blocks, 256, 0, st>>>(fpart, n_bins, nvr, L, p.maxp, fout, ld_fout)));
+      else
+        JSCC_TIMED("sc_finish_ratio", st,
+                   (sc_finish_ratio_kernel<2><<<blocks, 256, 0, st>>>(fpart, n_bins, nvr, L, p.maxp, row_idx, proj,
+                                                                      ld_proj, mode, floor_v, ratio, fout, ld_fout)));
+      JSCC_LAUNCH_CHECK();
+    }
+    if (stage == 1) return JSCC_OK;
+  } else if (stage != 2) {
     const size_t smem = Tr::kFwdRing + align_up((size_t)p.piece_cols * p.pitch * sizeof(float), 16);
     JSCC_CUDA_CHECK(allow_smem(sc_views_forward_kernel<T, NB, RING>));
     JSCC_TIMED("sc_views_forward", st,
@@ -648,7 +693,7 @@ static int sc_views(const T* A, int64_t lda, const int64_t* row_idx, int64_t n_b
   Carver cv(ws, ws_bytes);
   float* xt = cv.take<float>((size_t)V * p.pitch);
   float* ratio = cv.take<float>((size_t)n_bins * p.nb);
-  float* fpart = cv.take<float>((size_t)p.slices * n_bins * p.nb);
+  float* fpart = cv.take<float>(sv_forward_floats(p, n_bins));
   float* part = cv.take<float>((size_t)p.chunks * p.nb * (size_t)p.ldp);
   JSCC_REQUIRE(cv.ok(), "SC projector: workspace carve overflow");
   const int64_t cap = (int64_t)num_sms() * 16;
