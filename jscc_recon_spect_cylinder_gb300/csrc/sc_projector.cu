@@ -406,21 +406,27 @@ sc_colsum_kahan_kernel(const T* __restrict__ A, int64_t lda, const int64_t* __re
 
 // ------------------------------------------------------------------ reduce + inverse rotation
 // weight[j] += scale * sum_r sum_c part[c][r][src(j, r)] over the nr rotations of the block and their
-// chunks. A block takes 32 voxels; its eight warps each add one contiguous eighth of the (rotation,
-// chunk) terms and the eight sums are added in warp order (one fixed order), so the partial images are
-// read with eight times the loads in flight of one thread per voxel (bound by latency, not bytes: 76
-// images of 21,252 voxels 14.1 -> 8.0 us between events, of which about 5 are the events').
-constexpr int kRedWarps = 8;
+// chunks. SPLIT threads of a block share a voxel: each adds one contiguous part of the (rotation, chunk)
+// terms and the parts' sums are added in order (one fixed order), so the partial images are read with SPLIT
+// times the loads in flight of one thread per voxel (bound by latency, not bytes: 76 images of 21,252
+// voxels 14.1 -> 8.0 us between events, of which about 5 are the events'). Eight threads where the voxels are
+// few; from kRedFewVoxels on four, as eight then fill the chip's threads by themselves (back projection of
+// 1,777 BF16 rows, split 8 / 4 / 2: 36,000 voxels 29.9 / 27.8 / 27.8 us, weight of 5,555 87.0 / 86.2 / 87.6;
+// 14,400 voxels 154.5 / 155.3 / 156.8).
+constexpr int kRedThreads = 256;
+constexpr int64_t kRedFewVoxels = 24000;
 
-__global__ void __launch_bounds__(kRedWarps * 32)
+template <int SPLIT>
+__global__ void __launch_bounds__(kRedThreads)
 sc_reduce_scatter_kernel(const float* __restrict__ part, int64_t ldp, int chunks, int nr, int rb_stride,
                          const int64_t* __restrict__ rotinv, int64_t ld_rot, int r0, int64_t V, int has_scale,
                          float scale, float* __restrict__ weight) {
-  __shared__ float red[kRedWarps][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t j = (int64_t)blockIdx.x * 32 + lane;
+  constexpr int VOX = kRedThreads / SPLIT;  // voxels of a block
+  __shared__ float red[SPLIT][VOX];
+  const int vox = threadIdx.x % VOX, share = threadIdx.x / VOX;
+  const int64_t j = (int64_t)blockIdx.x * VOX + vox;
   const int terms = nr * chunks;
-  const int t0 = (int)((int64_t)terms * warp / kRedWarps), t1 = (int)((int64_t)terms * (warp + 1) / kRedWarps);
+  const int t0 = (int)((int64_t)terms * share / SPLIT), t1 = (int)((int64_t)terms * (share + 1) / SPLIT);
   float s = 0.f;
   if (j < V) {
     for (int t = t0; t < t1;) {
@@ -429,7 +435,7 @@ sc_reduce_scatter_kernel(const float* __restrict__ part, int64_t ldp, int chunks
       int64_t src = j;
       if (rotinv != nullptr) src = rotinv[j * ld_rot + r0 + r] - 1;
       if (src < 0 || src >= V) {
-        if (c_begin == 0) atomicAdd(&g_bad_index_count, 1u);  // counted by the warp that starts the rotation
+        if (c_begin == 0) atomicAdd(&g_bad_index_count, 1u);  // counted by the share that starts the rotation
       } else {
 #pragma unroll 8
         for (int c = c_begin; c < c_end; ++c) s += part[((int64_t)c * rb_stride + r) * ldp + src];
@@ -437,20 +443,27 @@ sc_reduce_scatter_kernel(const float* __restrict__ part, int64_t ldp, int chunks
       t += c_end - c_begin;
     }
   }
-  red[warp][lane] = s;
-  __syncthreads();
-  if (warp != 0 || j >= V) return;
+  if constexpr (SPLIT > 1) {
+    red[share][vox] = s;
+    __syncthreads();
+  }
+  if (share != 0 || j >= V) return;
 #pragma unroll
-  for (int w = 1; w < kRedWarps; ++w) s += red[w][lane];
+  for (int w = 1; w < SPLIT; ++w) s += red[w][vox];
   weight[j] = has_scale ? __fadd_rn(weight[j], __fmul_rn(scale, s)) : __fadd_rn(weight[j], s);
 }
 
 int launch_reduce_scatter(const float* part, int64_t ldp, int chunks, int nr, int rb_stride, const int64_t* rotinv,
                           int64_t ld_rot, int r0, int64_t V, int has_scale, float scale, float* weight,
                           cudaStream_t st) {
-  JSCC_TIMED("sc_reduce_scatter", st,
-             (sc_reduce_scatter_kernel<<<(unsigned)((V + 31) / 32), kRedWarps * 32, 0, st>>>(
-                 part, ldp, chunks, nr, rb_stride, rotinv, ld_rot, r0, V, has_scale, scale, weight)));
+  auto launch = [&](auto kernel, int split) {
+    const int vox = kRedThreads / split;
+    JSCC_TIMED("sc_reduce_scatter", st,
+               (kernel<<<(unsigned)((V + vox - 1) / vox), kRedThreads, 0, st>>>(
+                   part, ldp, chunks, nr, rb_stride, rotinv, ld_rot, r0, V, has_scale, scale, weight)));
+  };
+  if (V < kRedFewVoxels) launch(sc_reduce_scatter_kernel<8>, 8);
+  else launch(sc_reduce_scatter_kernel<4>, 4);
   JSCC_LAUNCH_CHECK();
   return JSCC_OK;
 }
