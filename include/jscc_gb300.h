@@ -466,11 +466,12 @@ JSCC_API int jscc_sparse_weight_split(const int32_t* row_id, const void* t_coars
  * and only read when have_sums != 0 (S_i depends on the rows, the sysmat and the grouping
  * only, so callers keep it across iterations with the same `order`). The coarse grid must fit in
  * shared memory (V_c floats <= 227 KB). Deterministic (fixed-order reductions).
- * For coarse grids of at most 9,600 voxels the weight runs as three bulk-copy pipelines, with
- * rows of any alignment (fastest: split rows whose starts are 16-byte aligned and whose pitch
- * ld_tc covers the row rounded up to whole 16-byte units, the values past V_c being anything)
- * and, for the first and the last, a 16-byte aligned sysmat row pitch: the group adjoints b_g (sysmat row segments streamed into shared memory), the event coefficients and
- * q_g (b_g and the coarse rows streamed in), and the scatter (sysmat tiles and q segments
+ * For coarse grids of at most 9,600 voxels the weight runs as three bulk-copy pipelines: with split
+ * rows whose starts are 16-byte aligned and whose pitch ld_tc covers the row rounded up to whole
+ * 16-byte units (the values past V_c being anything), and with other rows where grid, taps and
+ * groups are large enough for it to pay; the first and the last need a 16-byte aligned sysmat row
+ * pitch. They are the group adjoints b_g (sysmat row segments streamed into shared memory), the event
+ * coefficients and q_g (b_g and the coarse rows streamed in), and the scatter (sysmat tiles and q segments
  * streamed in); their waits are bounded and a wait that gives up is counted
  * (jscc_take_wait_timeout_count), the weight of that call then being invalid.
  * ring_len / ring_stride (0 / 0: no claim) state that the adjoint table is a stride-4 ring

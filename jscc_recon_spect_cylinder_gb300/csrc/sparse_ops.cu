@@ -740,6 +740,7 @@ sparse_group_coef_kernel(SpRows<TC> rows, bool vec_rows, const int32_t* __restri
 // Every wait is bounded: on a timeout the CTA counts it (jscc_take_wait_timeout_count),
 // waits (bounded) for the copies it still has in flight and returns.
 constexpr int kBkThreads = 512;
+constexpr int64_t kBkFewEvents = 200;
 constexpr int kBkEventWarps = 15;
 constexpr int kBkEvents = kBkEventWarps * 32;
 constexpr int kBkProducerWarp = kBkEventWarps;
@@ -2265,7 +2266,21 @@ static int grouped_launch(const SpRows<TC>& rows, bool vec_rows, int64_t n_event
   // events of a chunk: a power of two leaving as many slots in flight as it holds
   int batch = 1;
   while (batch * 2 <= kBkMaxBatch && batch * 2 <= n_slots / 2) batch *= 2;
-  const bool bulk = n_slots >= 2 && vc <= kBkMaxCoarse && ldq % 4 == 0;
+  // Rows in the LOOSE form, and grids whose sysmat rows are not whole 16-byte units on 16-byte boundaries,
+  // take it where it pays: an exchange over the CTA for up to four events costs about as much as the general kernel
+  // spends on 1,500 to 3,000 coarse values, and that kernel's adjoint grows with the taps. 20,000 events
+  // in 4,000 groups, bulk against general: packed rows, 7 taps, 300 voxels 172 and 92 us, 1,200 voxels 191 and
+  // 214, 2,700 voxels 231 and 408; 3 taps, 1,380 voxels 248 and 197, 2,400 voxels 278 and 273, 5,400 voxels 372
+  // and 490; unaligned BF16 rows, 3 taps, 2,400 voxels 294 and 261, 5,400 voxels 386 and 422; 1 tap, 3,825
+  // voxels 249 and 233, in 400 groups 136 and 259. Small grids with many taps lose it again when a group's events
+  // outweigh its adjoint (56 taps, 480 voxels: 4,000 groups 213 and 375 us, 400 groups 134 and 107). Below
+  // kBkFewEvents either is a few launches long (300 events, 300 voxels: 23 and 16 us).
+  const bool whole = !loose && reinterpret_cast<uintptr_t>(eff) % 16 == 0 && (ld_eff * sizeof(TE)) % 16 == 0 &&
+                     ((size_t)vf * sizeof(TE)) % 16 == 0;
+  const bool many = n_events >= 16 * (int64_t)n_groups;
+  const int64_t reach = vc * (K + 5);
+  const bool pays = whole || n_events < kBkFewEvents || (reach >= (sizeof(TC) == 4 || many ? 20000 : 25000) && !(vc < 1000 && many));
+  const bool bulk = pays && n_slots >= 2 && vc <= kBkMaxCoarse && ldq % 4 == 0;
   const size_t bk_smem = (size_t)slot_off + (size_t)n_slots * slot_stride;
   int64_t bk_grid = num_sms();
   if (bk_grid > n_groups) bk_grid = n_groups;
