@@ -412,9 +412,9 @@ class _Workspace:
         finally:
             self._owner.buffers = outer
 
-    def get(self, device: torch.device, nbytes: int, at_least: int | None = None) -> torch.Tensor:
+    def get(self, device: torch.device, nbytes: int, at_least=None) -> torch.Tensor:
         """At least ``nbytes`` of scratch; where they cannot be had and the caller can work in less,
-        ``at_least`` of them (a request that failed is not tried again before ``clear``: each trial
+        ``at_least`` of them, a number or a function that says it (a request that failed is not tried again before ``clear``: each trial
         would wait for the device and empty torch's cache)."""
         own = getattr(self._owner, "buffers", None)
         if own is not None:
@@ -425,7 +425,7 @@ class _Workspace:
             self._captured.add(key)
         buf = self._bufs.get(key)
         if at_least is not None and nbytes >= self._refused.get(key, nbytes + 1):
-            nbytes = at_least
+            nbytes, at_least = at_least() if callable(at_least) else at_least, None
         if buf is not None and buf.numel() >= nbytes:
             return buf
         size = nbytes
@@ -434,24 +434,26 @@ class _Workspace:
         try:
             new = torch.empty(max(size, 256), dtype=torch.uint8, device=device)
         except torch.OutOfMemoryError:
-            if at_least is None or at_least >= nbytes:
+            least = at_least() if callable(at_least) else at_least
+            if least is None or least >= nbytes:
                 raise
             self._refused[key] = nbytes
-            return self.get(device, at_least)
+            return self.get(device, least)
         if buf is not None and key in self._captured:
             self._kept.append(buf)
         self._bufs[key] = new
         return new
 
     @staticmethod
-    def _grow_own(own: list, device: torch.device, nbytes: int, at_least: int | None) -> torch.Tensor:
+    def _grow_own(own: list, device: torch.device, nbytes: int, at_least) -> torch.Tensor:
         if not own or own[-1].numel() < nbytes:
             try:
                 own.append(torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device))
             except torch.OutOfMemoryError:
-                if at_least is None or at_least >= nbytes:
+                least = at_least() if callable(at_least) else at_least
+                if least is None or least >= nbytes:
                     raise
-                return _Workspace._grow_own(own, device, at_least, None)
+                return _Workspace._grow_own(own, device, least, None)
         return own[-1]
 
     def clear(self) -> None:

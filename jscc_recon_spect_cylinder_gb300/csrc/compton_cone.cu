@@ -1051,7 +1051,8 @@ struct ConePlan {
 constexpr int kConeFwdCtas = 5;                       // resident forward CTAs an SM
 constexpr size_t kConeStoreMax = (size_t)1 << 30;   // stored rows: at most this much workspace
 
-static ConePlan plan_cone(int64_t n_ev, int64_t V) {
+// `rows`: for a call that stores rows (their plan costs the host more than all the rest)
+static ConePlan plan_cone(int64_t n_ev, int64_t V, bool rows) {
   ConePlan p{};
   const int64_t tiles = (V + kConeThreads - 1) / kConeThreads;
   const int64_t target = 2432;  // back-pass CTAs: 16 x 152 SMs
@@ -1077,7 +1078,7 @@ static ConePlan plan_cone(int64_t n_ev, int64_t V) {
   if (stages > 65535) stages = 65535;
   const int64_t fit = stages * kRowsStage;
   p.store_ev = n_ev < fit ? n_ev : fit;
-  if (p.store_ev > 0) {
+  if (rows && p.store_ev > 0) {
     p.sc_bytes = rows_weight_bytes(p.store_ev, V);
     p.store_bytes = align_up((size_t)p.store_ev * p.ldp * sizeof(float), 256) + align_up(p.sc_bytes, 256) + 512;
   }
@@ -1322,12 +1323,15 @@ int jscc_compton_row_stats(const float* records, const int32_t* row_id, int64_t 
 }
 
 size_t jscc_compton_weight_workspace_bytes(int64_t n_ev, int64_t n_vox) {
-  const ConePlan p = plan_cone(n_ev, n_vox);
+  const ConePlan p = plan_cone(n_ev, n_vox, true);
   return p.ws_bytes + (p.store_bytes > p.slice_bytes ? p.store_bytes : p.slice_bytes);
 }
 
 // What a call uses beyond the minimum: the strict weight over every pair stores rows, the strict
 // projection over every pair has slices; nothing else does either.
+static bool cone_stores_rows(int stage, int32_t model, int32_t use_window) {
+  return stage == 0 && model == JSCC_CONE_STRICT && !use_window;
+}
 static size_t cone_more_bytes(const ConePlan& p, int stage, int32_t model, int32_t use_window) {
   if (model != JSCC_CONE_STRICT || use_window) return 0;
   return stage == 0 ? p.store_bytes : stage == 1 ? p.slice_bytes : 0;
@@ -1335,7 +1339,7 @@ static size_t cone_more_bytes(const ConePlan& p, int stage, int32_t model, int32
 
 size_t jscc_compton_workspace_bytes(int64_t n_ev, int64_t n_vox, int32_t call, int32_t model, int32_t use_window,
                                     int32_t preferred) {
-  const ConePlan p = plan_cone(n_ev, n_vox);
+  const ConePlan p = plan_cone(n_ev, n_vox, preferred && cone_stores_rows(call, model, use_window));
   return p.ws_bytes + (preferred ? cone_more_bytes(p, call, model, use_window) : 0);
 }
 
@@ -1360,7 +1364,7 @@ static int compton_stage_entry(const char* what, int stage, const float* records
   JSCC_REQUIRE(stage != 2 || g, "%s: null input", what);
   JSCC_REQUIRE(!eff || (row_id && ld_eff >= n_vox), "%s: efficiency rows need row ids, ld >= V", what);
   JSCC_REQUIRE(stage != 0 || (rotmat == nullptr) == (rotmat_inv == nullptr), "%s: give both rotation tables", what);
-  const ConePlan p = plan_cone(n_ev, n_vox);
+  const ConePlan p = plan_cone(n_ev, n_vox, cone_stores_rows(stage, model, use_window));
   JSCC_REQUIRE(workspace && workspace_bytes >= p.ws_bytes, "%s: workspace too small (%zu < %zu)", what,
                workspace_bytes, p.ws_bytes);
   Carver cv(workspace, workspace_bytes);
@@ -1435,8 +1439,7 @@ int jscc_compton_weight(const float* records, const int32_t* row_id, int64_t n_e
 }
 
 size_t jscc_compton_loglik_workspace_bytes(int64_t n_ev, int64_t n_vox) {
-  const ConePlan p = plan_cone(n_ev, n_vox);
-  return p.store_bytes;
+  return plan_cone(n_ev, n_vox, true).store_bytes;
 }
 
 int jscc_compton_loglik(const float* records, const int32_t* row_id, int64_t n_ev, const float* coor, int64_t n_vox,
@@ -1448,7 +1451,7 @@ int jscc_compton_loglik(const float* records, const int32_t* row_id, int64_t n_e
   if (n_ev == 0 || n_vox == 0) return JSCC_OK;
   JSCC_REQUIRE(records && row_id && coor && img && f && grad, "%s: null pointer argument", what);
   JSCC_REQUIRE(!eff || ld_eff >= n_vox, "%s: efficiency rows need ld >= V", what);
-  const ConePlan p = plan_cone(n_ev, n_vox);
+  const ConePlan p = plan_cone(n_ev, n_vox, true);
   JSCC_REQUIRE(p.store_ev > 0, "%s: too many voxels (%lld)", what, (long long)n_vox);
   JSCC_REQUIRE(workspace && workspace_bytes >= p.store_bytes, "%s: workspace too small (%zu < %zu)", what,
                workspace_bytes, p.store_bytes);

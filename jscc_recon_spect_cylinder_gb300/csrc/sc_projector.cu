@@ -694,8 +694,10 @@ static int sc_one_view(const T* A, int64_t lda, const int64_t* row_idx, int64_t 
 // One view takes the kernels of several views (padded to two) where they are the faster ones.
 // The weight: the fused kernel costs a row 8.7 + 0.2 V / 1000 ns, 13 + 0.3 V / 1000 with rows off
 // 16-byte boundaries, mostly its exchange, however short the row is; the two passes cost 1.5 V / 1000
-// (float32) or 1.3 V / 1000 ns (BF16) and two launches more, about 6 us (12,000 float32 rows of 1,440
-// voxels: 112 against 32 us; of 14,400 voxels: 136 against 280 us). The halves on their own: rows off
+// (float32) or 1.3 V / 1000 ns (BF16) and three launches more, about 6 us there and as much again where the
+// host's calls set the pace (12,000 float32 rows of 1,440 voxels: 112 against 32 us; of 14,400 voxels: 136
+// against 280 us; 1,400 rows of 1,024 voxels, a gain of 10 us by this count: 19.1 against 13.1 us in a graph, the
+// weight of as many listed events from Python 45 against 49 us). The halves on their own: rows off
 // 16-byte boundaries, which the one-view forward pass reads a value at a time.
 template <typename T>
 static bool one_view_by_views(const T* A, int64_t lda, int64_t n_bins, int64_t V, int stage) {
@@ -705,7 +707,7 @@ static bool one_view_by_views(const T* A, int64_t lda, int64_t n_bins, int64_t V
   const bool loose = !vec_ok || V % (16 / (int64_t)sizeof(T)) != 0;
   const double fused = loose ? 13.0 + 0.3 * k : 8.7 + 0.2 * k;
   const double views = (sizeof(T) == 4 ? 1.5 : 1.3) * k;
-  return (double)n_bins * (fused - views) > 6000.0;
+  return (double)n_bins * (fused - views) > 12000.0;
 }
 
 // The weight or one of its halves (stage as in sc_one_view) for any number of views, in a

@@ -236,8 +236,9 @@ def sc_backproject(sysmat, g, rotmat_inv=None, n_rot=None, row_idx=None, scale=1
 def _compton_scratch(lib, dev, n, V, call, model, use_window):
     """Scratch of a Compton call (0 weight, 1 project, 2 backproject): what it prefers (the strict weight:
     up to 1 GB of rows), or the least it takes where memory is short."""
-    want, least = (lib.jscc_compton_workspace_bytes(n, V, call, int(model), 1 if use_window else 0, p) for p in (1, 0))
-    return _lib.workspace.get(dev, want, least)
+    a = (n, V, call, int(model), 1 if use_window else 0)
+    return _lib.workspace.get(dev, lib.jscc_compton_workspace_bytes(*a, 1),
+                              lambda: lib.jscc_compton_workspace_bytes(*a, 0))
 
 
 def compton_project(records, row_id, coor, img, model=_lib.CONE_STRICT, eff=None, use_window=False, rotmat=None,
