@@ -23,8 +23,8 @@
 //     the efficiency load (K = window_sigmas; K <= 0 evaluates every pair).
 //   * Weight, strict model: the rows of a block of events (up to 1 GB of workspace) are evaluated
 //     once and stored, and the SC kernels weight them. With a window the passes evaluate instead: a
-//     pair outside it costs less than a stored value. So do the other models, and a workspace without
-//     room for the rows.
+//     pair outside it costs less than a stored value. So do the other models, short rows, and a
+//     workspace without room for the rows.
 //   * Forward: CTA = 256 threads x EB events; every thread walks voxels, keeps EB partial
 //     sums in registers, fixed-order CTA reduction at the end. A strict projection of few events
 //     takes several CTAs a block of events, a voxel slice each: 1,500 events x 36,000 voxels
@@ -1329,8 +1329,11 @@ size_t jscc_compton_weight_workspace_bytes(int64_t n_ev, int64_t n_vox) {
 
 // What a call uses beyond the minimum: the strict weight over every pair stores rows, the strict
 // projection over every pair has slices; nothing else does either.
-static bool cone_stores_rows(int stage, int32_t model, int32_t use_window) {
-  return stage == 0 && model == JSCC_CONE_STRICT && !use_window;
+// (Short rows cost the SC kernel more than their second evaluation: 1,500 events on 600 voxels 25 us evaluated
+// twice, 40 stored, on 1,200 voxels 31 and 40, on 2,400 47 and 41; 6,000 events on 600 voxels 34 and 43, on
+// 1,200 54 and 46.)
+static bool cone_stores_rows(int stage, int32_t model, int32_t use_window, int64_t n_ev, int64_t V) {
+  return stage == 0 && model == JSCC_CONE_STRICT && !use_window && (V >= 2000 || (V >= 1000 && n_ev >= 3000));
 }
 static size_t cone_more_bytes(const ConePlan& p, int stage, int32_t model, int32_t use_window) {
   if (model != JSCC_CONE_STRICT || use_window) return 0;
@@ -1339,7 +1342,7 @@ static size_t cone_more_bytes(const ConePlan& p, int stage, int32_t model, int32
 
 size_t jscc_compton_workspace_bytes(int64_t n_ev, int64_t n_vox, int32_t call, int32_t model, int32_t use_window,
                                     int32_t preferred) {
-  const ConePlan p = plan_cone(n_ev, n_vox, preferred && cone_stores_rows(call, model, use_window));
+  const ConePlan p = plan_cone(n_ev, n_vox, preferred && cone_stores_rows(call, model, use_window, n_ev, n_vox));
   return p.ws_bytes + (preferred ? cone_more_bytes(p, call, model, use_window) : 0);
 }
 
@@ -1364,7 +1367,7 @@ static int compton_stage_entry(const char* what, int stage, const float* records
   JSCC_REQUIRE(stage != 2 || g, "%s: null input", what);
   JSCC_REQUIRE(!eff || (row_id && ld_eff >= n_vox), "%s: efficiency rows need row ids, ld >= V", what);
   JSCC_REQUIRE(stage != 0 || (rotmat == nullptr) == (rotmat_inv == nullptr), "%s: give both rotation tables", what);
-  const ConePlan p = plan_cone(n_ev, n_vox, cone_stores_rows(stage, model, use_window));
+  const ConePlan p = plan_cone(n_ev, n_vox, cone_stores_rows(stage, model, use_window, n_ev, n_vox));
   JSCC_REQUIRE(workspace && workspace_bytes >= p.ws_bytes, "%s: workspace too small (%zu < %zu)", what,
                workspace_bytes, p.ws_bytes);
   Carver cv(workspace, workspace_bytes);
@@ -1392,7 +1395,7 @@ static int compton_stage_entry(const char* what, int stage, const float* records
   }
   int rc;
   const bool win = use_window != 0 && model == JSCC_CONE_STRICT;
-  if (stage == 0 && model == JSCC_CONE_STRICT && !win && more != nullptr && p.store_ev > 0)
+  if (stage == 0 && more != nullptr)
     return eff_dtype == JSCC_DTYPE_F32
                ? launch_cone_stored<float>(rec, row_id, n_ev, coor, n_vox, x, static_cast<const float*>(eff), ld_eff,
                                            rotmat_inv, ld_rot, kRatio, 0.f, scale, weight, nullptr, p, more, st)
