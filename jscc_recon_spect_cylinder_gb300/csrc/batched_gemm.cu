@@ -258,6 +258,7 @@ bf16_gemm_nt_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_consta
       if (lane == 0) mbar_arrive(&acc_free[seg & 1]);
     }
   }
+  __syncwarp();  // a role's idle lanes wait here: polling beside it they took turns with its own instructions
   if (nk > 0) ok = role_wait(done, 0u, abort_flag, polls) && ok && !*abort_flag;
   ok = __syncthreads_and(ok);  // every role has left its loop: nothing more is issued
   if (!ok && tid == 0) {
