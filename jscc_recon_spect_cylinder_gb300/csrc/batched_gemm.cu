@@ -14,8 +14,11 @@
 // GEMM kernel (one CTA per row tile and K split, warp-specialised). Bound by the bytes of P; what it
 // needs for that is R read from L2 seldom enough and enough copies in flight. 65-128 columns take tiles
 // of 256 rows, one CTA an SM: two accumulators share each R tile, which tiles of 128 rows would read
-// twice as often. Up to 64 columns R is small, and tiles of 128 rows, two CTAs an SM, split the rows
-// more evenly; above 128 columns the accumulators of 128 rows fill TMEM.
+// twice as often. Where tiles of 128 rows number no more than the SMs, those take them: twice the CTAs, each
+// bound by the latency of its own chain of K steps (4,096 x 36,000 by 128 in one split 282 us with tiles
+// of 256 rows, 202 us so, in four 87 and 67 us; in eight 69 us with tiles of 256 rows). Up to 64 columns R is
+// small, and tiles of 128 rows, two CTAs an SM, split the rows more evenly; above 128 columns the
+// accumulators of 128 rows fill TMEM.
 //   * producer (first warp after the adders, one thread): TMA tiled loads (cp.async.bulk.tensor, 128-byte swizzle)
 //     of the P and R tiles of each 64-wide K step into a ring of shared-memory stages, each
 //     completing on the stage's "full" mbarrier (expect-tx bytes);
@@ -125,12 +128,13 @@ __device__ __forceinline__ bool role_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
-template <int NR>
+template <int NR, int TILES>
 struct GemmCfg {
   static_assert(NR == 32 || NR == 64 || NR == 128 || NR == 256, "MMA N for M = 128, columns a power of 2");
-  static constexpr int kGroups = NR <= 64 ? 1 : 2;       // groups of four adder warps
-  static constexpr int kTiles = NR == 128 ? 2 : 1;       // 128-row tiles of a CTA
+  static_assert(TILES == 1 || NR == 128, "two accumulators in TMEM");
+  static constexpr int kTiles = TILES;                   // 128-row tiles of a CTA
   static constexpr int kCols = NR == 256 ? 128 : NR;     // columns of a group
+  static constexpr int kGroups = NR == 256 ? 2 : TILES;  // groups of four adder warps
   static constexpr int kCtas = NR <= 64 ? 2 : 1;         // an SM
   static constexpr int kAdders = 128 * kGroups;
   static constexpr int kThreads = kAdders + 64;
@@ -146,12 +150,12 @@ struct GemmCfg {
 };
 
 // out[split][m][n] = sum_{k in split} P[m, k] R[n, k]   (rows m < M, n < nr; FP32)
-template <int NR>
-__global__ void __launch_bounds__(GemmCfg<NR>::kThreads, GemmCfg<NR>::kCtas)
+template <int NR, int TILES>
+__global__ void __launch_bounds__(GemmCfg<NR, TILES>::kThreads, GemmCfg<NR, TILES>::kCtas)
 bf16_gemm_nt_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmR, int64_t M,
                     int nr, int64_t K, int64_t k_per_split, float* __restrict__ out, int64_t ldo,
                     int64_t split_stride, int vec4) {
-  using C = GemmCfg<NR>;
+  using C = GemmCfg<NR, TILES>;
   constexpr int S = C::kStages, W = C::kCols, SET = C::kGroups * W, AW = C::kAdders / 32;
   extern __shared__ uint8_t gsm_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~uintptr_t(1023));
@@ -477,10 +481,10 @@ bool make_map(CUtensorMap* map, const void* base, int64_t K, int64_t rows, int64
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int NR>
+template <int NR, int TILES>
 int launch_gemm(const __nv_bfloat16* P, int64_t ldp, const __nv_bfloat16* R, int64_t ldr, int64_t M, int nr, int64_t K,
                 int splits, float* out, int64_t ldo, float* part, cudaStream_t st) {
-  using C = GemmCfg<NR>;
+  using C = GemmCfg<NR, TILES>;
   // the shared-memory attribute is set once per device (outside any later graph capture: the
   // first call on a device happens eagerly)
   static std::atomic<unsigned long long> attr_set{0};
@@ -488,8 +492,8 @@ int launch_gemm(const __nv_bfloat16* P, int64_t ldp, const __nv_bfloat16* R, int
   JSCC_CUDA_CHECK(cudaGetDevice(&dev));
   const unsigned long long bit = 1ull << (dev & 63);
   if (!(attr_set.load() & bit)) {
-    JSCC_CUDA_CHECK(cudaFuncSetAttribute(bf16_gemm_nt_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)C::kSmem));
+    JSCC_CUDA_CHECK(cudaFuncSetAttribute(bf16_gemm_nt_kernel<NR, TILES>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem));
     attr_set.fetch_or(bit);
   }
   int64_t kps = (K + splits - 1) / splits;
@@ -511,7 +515,8 @@ int launch_gemm(const __nv_bfloat16* P, int64_t ldp, const __nv_bfloat16* R, int
   const int64_t sstride = used > 1 ? M * nr : 0;
   const int vec4 = nr % 4 == 0 && ldd % 4 == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0;
   JSCC_TIMED("bf16_gemm_nt", st,
-             (bf16_gemm_nt_kernel<NR><<<grid, C::kThreads, C::kSmem, st>>>(mp, mr, M, nr, K, kps, dst, ldd, sstride, vec4)));
+             (bf16_gemm_nt_kernel<NR, TILES><<<grid, C::kThreads, C::kSmem, st>>>(mp, mr, M, nr, K, kps, dst, ldd, sstride,
+                                                                              vec4)));
   JSCC_LAUNCH_CHECK();
   if (used > 1) {
     int64_t blocks = (M * nr + 255) / 256;
@@ -563,10 +568,12 @@ int jscc_bf16_gemm_nt(const void* P, int64_t ldp, const void* R, int64_t ldr, in
   const auto* r = static_cast<const __nv_bfloat16*>(R);
   float* part = static_cast<float*>(workspace);
   cudaStream_t st = as_stream(stream);
-  if (nr <= 32) return launch_gemm<32>(p, ldp, r, ldr, M, nr, K, k_splits, out, ldo, part, st);
-  if (nr <= 64) return launch_gemm<64>(p, ldp, r, ldr, M, nr, K, k_splits, out, ldo, part, st);
-  if (nr <= 128) return launch_gemm<128>(p, ldp, r, ldr, M, nr, K, k_splits, out, ldo, part, st);
-  return launch_gemm<256>(p, ldp, r, ldr, M, nr, K, k_splits, out, ldo, part, st);
+  auto launch = [&](auto fn) { return fn(p, ldp, r, ldr, M, nr, K, k_splits, out, ldo, part, st); };
+  if (nr <= 32) return launch(launch_gemm<32, 1>);
+  if (nr <= 64) return launch(launch_gemm<64, 1>);
+  const bool few = (M + kGM - 1) / kGM * k_splits <= num_sms();
+  if (nr <= 128) return few ? launch(launch_gemm<128, 1>) : launch(launch_gemm<128, 2>);
+  return launch(launch_gemm<256, 1>);
 }
 
 int jscc_batch_split(const float* x, int64_t ldx, int32_t n_inst, int32_t np, int64_t V, void* xs, int64_t ldxs,
