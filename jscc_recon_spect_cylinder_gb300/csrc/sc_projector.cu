@@ -721,7 +721,7 @@ static int sc_run(const T* A, int64_t lda, const int64_t* row_idx, int64_t n_bin
   const int has_scale = scale != 1.0f;
   // (one view in less than its padding to two takes goes the way that the smallest workspace is made for)
   if (n_rot > 1 || (one_view_by_views<T>(A, lda, n_bins, V, stage) &&
-                    plan_views(n_bins, V, 1, ws_bytes, sizeof(T)).bytes <= ws_bytes))
+                    plan_views(n_bins, V, 1, ws_bytes, sizeof(T), sv_aligned(A, lda)).bytes <= ws_bytes))
     return sc_views<T>(A, lda, row_idx, n_bins, V, proj, ld_proj, n_rot, img, rotmat, rotinv, ld_rot, mode,
                        floor_v, has_scale, scale, weight, ws, ws_bytes, st, stage, fout, ld_fout, gin, ld_gin);
   Carver cv(ws, ws_bytes);
@@ -896,8 +896,9 @@ size_t jscc_sc_weight_workspace_bytes(int64_t n_bins, int64_t n_vox, int32_t n_r
   const size_t one = p.ws_bytes + p.fs_bytes;
   if (n_rot < 1 || n_bins < 1 || n_vox < 1) return one;
   size_t most = one;
-  for (size_t el : {sizeof(float), sizeof(__nv_bfloat16)}) {
-    const size_t views = plan_views(n_bins, n_vox, n_rot, SIZE_MAX, el).bytes;
+  for (int form = 0; form < 3; ++form) {  // float32, BF16, BF16 off 16-byte boundaries
+    const size_t el = form == 0 ? sizeof(float) : sizeof(__nv_bfloat16);
+    const size_t views = plan_views(n_bins, n_vox, n_rot, SIZE_MAX, el, form < 2).bytes;
     if (views > most) most = views;
   }
   return most;

@@ -532,7 +532,12 @@ static size_t sv_bytes(const SvPlan& p, int64_t n_bins, int64_t V) {
   return b + 256;
 }
 
-static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap, size_t el) {
+template <typename T>
+static bool sv_aligned(const T* A, int64_t lda) {
+  return (lda * (int64_t)sizeof(T)) % 16 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
+}
+
+static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap, size_t el, bool aligned) {
   const int64_t sms = num_sms();
   SvPlan p{};
   p.ldp = (int64_t)align_up((size_t)V, 8);
@@ -558,7 +563,7 @@ static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap, size_
     if (slices < want) slices = want;
     if (slices > units) slices = units;
     // back: about two CTAs an SM, at least eight rows a warp
-    const int64_t tile = sv_back_cols(p.nb, el, true), tiles = (V + tile - 1) / tile;
+    const int64_t tile = sv_back_cols(p.nb, el, aligned), tiles = (V + tile - 1) / tile;
     const int64_t most = (n_bins + 63) / 64;
     int64_t chunks = (2 * sms + tiles - 1) / tiles;
     if (chunks > most) chunks = most;
@@ -621,7 +626,7 @@ static int sv_launch_block(const T* A, int64_t lda, const int64_t* row_idx, int6
                            const float* proj, int64_t ld_proj, int mode, float floor_v, int stage, float* fout,
                            int64_t ld_fout, cudaStream_t st) {
   using Tr = SvTraits<T, NB, RING>;
-  const bool split = NB == 2 && sizeof(T) == 4 && p.ranges > 0 && lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
+  const bool split = NB == 2 && sizeof(T) == 4 && p.ranges > 0 && sv_aligned(A, lda);
   if (stage != 2 && split) {
     if constexpr (NB == 2 && sizeof(T) == 4) {
       const int64_t nvr = (V + 3) / 4, L = (n_bins * nvr + p.ranges - 1) / p.ranges;
@@ -687,7 +692,7 @@ static int sc_views(const T* A, int64_t lda, const int64_t* row_idx, int64_t n_b
                     int64_t ld_rot, int mode, float floor_v, int has_scale, float scale, float* weight,
                     void* ws, size_t ws_bytes, cudaStream_t st, int stage, float* fout, int64_t ld_fout,
                     const float* gin, int64_t ld_gin) {
-  const SvPlan p = plan_views(n_bins, V, n_rot, ws_bytes, sizeof(T));
+  const SvPlan p = plan_views(n_bins, V, n_rot, ws_bytes, sizeof(T), sv_aligned(A, lda));
   JSCC_REQUIRE(p.bytes <= ws_bytes, "SC projector: %d views need %zu bytes of workspace (%zu given)", n_rot, p.bytes,
                ws_bytes);
   Carver cv(ws, ws_bytes);
