@@ -693,21 +693,24 @@ static int sc_one_view(const T* A, int64_t lda, const int64_t* row_idx, int64_t 
 
 // One view takes the kernels of several views (padded to two) where they are the faster ones.
 // The weight: the fused kernel costs a row 8.7 + 0.2 V / 1000 ns, 13 + 0.3 V / 1000 with rows off
-// 16-byte boundaries, mostly its exchange, however short the row is; the two passes cost 1.5 V / 1000
-// (float32) or 1.3 V / 1000 ns (BF16) and three launches more, about 6 us there and as much again where the
-// host's calls set the pace (12,000 float32 rows of 1,440 voxels: 112 against 32 us; of 14,400 voxels: 136
-// against 280 us; 1,400 rows of 1,024 voxels, a gain of 10 us by this count: 19.1 against 13.1 us in a graph, the
-// weight of as many listed events from Python 45 against 49 us). The halves on their own: rows off
-// 16-byte boundaries, which the one-view forward pass reads a value at a time.
+// 16-byte boundaries, mostly its exchange, however short the row is; the two passes cost 1.7 V / 1000
+// (float32; 2.25 for aligned rows taken by their ids, out of order) or 1.3 V / 1000 ns (BF16) and three
+// launches more: about 6 us there, and as much again in updates short enough (up to about 45 us) for the host
+// to set their pace: two joint subsets of 3,280 BF16 rows of 5,440 voxels 237 us so, 217 us with the fused
+// kernel, though that is 9 us slower by itself. Rows off 16-byte boundaries: 693 float32 rows of 1,441 voxels 17.5 against 11.8 us. 12,000 float32 rows of 1,440 voxels: 114 against 34 us; of 5,280 voxels 120
+// against 108, by their ids 126 against 135; of 8,000 voxels 127 against 162; BF16 128 against 66 us of 5,280
+// voxels, 131 against 93 of 8,000. The halves on their own: rows off 16-byte boundaries, which the one-view
+// forward pass reads a value at a time.
 template <typename T>
-static bool one_view_by_views(const T* A, int64_t lda, int64_t n_bins, int64_t V, int stage) {
+static bool one_view_by_views(const T* A, int64_t lda, bool ids, int64_t n_bins, int64_t V, int stage) {
   const bool vec_ok = (lda * (int64_t)sizeof(T)) % 16 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
   if (stage != 0) return !vec_ok;
   const double k = (double)V / 1000.0;
   const bool loose = !vec_ok || V % (16 / (int64_t)sizeof(T)) != 0;
   const double fused = loose ? 13.0 + 0.3 * k : 8.7 + 0.2 * k;
-  const double views = (sizeof(T) == 4 ? 1.5 : 1.3) * k;
-  return (double)n_bins * (fused - views) > 12000.0;
+  const double views = (sizeof(T) == 2 ? 1.3 : ids && !loose ? 2.25 : 1.7) * k;
+  const double gain = (double)n_bins * (fused - views);
+  return gain > (loose || (double)n_bins * fused > 45000.0 ? 6000.0 : 12000.0);
 }
 
 // The weight or one of its halves (stage as in sc_one_view) for any number of views, in a
@@ -720,7 +723,7 @@ static int sc_run(const T* A, int64_t lda, const int64_t* row_idx, int64_t n_bin
                   int64_t ld_gin) {
   const int has_scale = scale != 1.0f;
   // (one view in less than its padding to two takes goes the way that the smallest workspace is made for)
-  if (n_rot > 1 || (one_view_by_views<T>(A, lda, n_bins, V, stage) &&
+  if (n_rot > 1 || (one_view_by_views<T>(A, lda, row_idx != nullptr, n_bins, V, stage) &&
                     plan_views(n_bins, V, 1, ws_bytes, sizeof(T), sv_aligned(A, lda)).bytes <= ws_bytes))
     return sc_views<T>(A, lda, row_idx, n_bins, V, proj, ld_proj, n_rot, img, rotmat, rotinv, ld_rot, mode,
                        floor_v, has_scale, scale, weight, ws, ws_bytes, st, stage, fout, ld_fout, gin, ld_gin);
