@@ -2333,8 +2333,10 @@ static int grouped_launch(const SpRows<TC>& rows, bool vec_rows, int64_t n_event
   }
   // the stencil times several z taps, one ring a plane (the radially coarsened grid): tiles of whole
   // coarse rings, one voxel per compute thread, about one CTA an SM
+  // (few groups gather their taps: 243 groups on 480 coarse voxels, 56 taps, 30 against 35 us for the weight, 2,800
+  // groups 174 against 103)
   const int n_z = K / 7;
-  const bool zring = bulk && !ring && reinterpret_cast<uintptr_t>(eff) % 16 == 0 && (ld_eff * sizeof(TE)) % 16 == 0 &&
+  const bool zring = bulk && !ring && (int64_t)n_groups * vc >= 250000 && reinterpret_cast<uintptr_t>(eff) % 16 == 0 && (ld_eff * sizeof(TE)) % 16 == 0 &&
                      ((size_t)vf * sizeof(TE)) % 16 == 0 && ring_stride == 4 && K % 7 == 0 && n_z <= 8 &&
                      ring_len >= 8 && taps.n_lf == ring_len && taps.n_lc * 4 == ring_len && taps.n_lc <= kAzThreads &&
                      vf < (1 << 30);
