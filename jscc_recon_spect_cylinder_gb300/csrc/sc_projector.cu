@@ -898,13 +898,8 @@ size_t jscc_sc_weight_workspace_bytes(int64_t n_bins, int64_t n_vox, int32_t n_r
   const ScPlan p = plan_sc(n_bins, n_vox, n_rot);
   const size_t one = p.ws_bytes + p.fs_bytes;
   if (n_rot < 1 || n_bins < 1 || n_vox < 1) return one;
-  size_t most = one;
-  for (int form = 0; form < 3; ++form) {  // float32, BF16, BF16 off 16-byte boundaries
-    const size_t el = form == 0 ? sizeof(float) : sizeof(__nv_bfloat16);
-    const size_t views = plan_views(n_bins, n_vox, n_rot, SIZE_MAX, el, form < 2).bytes;
-    if (views > most) most = views;
-  }
-  return most;
+  const size_t views = plan_views(n_bins, n_vox, n_rot, SIZE_MAX, 0, true).bytes;
+  return views > one ? views : one;
 }
 
 int jscc_sc_weight(const void* A, int32_t a_dtype, int64_t lda, const int64_t* row_idx,

@@ -518,6 +518,7 @@ struct SvPlan {
 // is for BF16, of three views on, and past 25,600 voxels (2,777 x 36,000: 87 against 95 us).
 constexpr int64_t kSvSplitBytes = 96000000;
 constexpr size_t kSvSplitSmem = 200 * 1024;
+constexpr double kSvPlanBytes = 24e6;  // smaller matrices: the host's time for the search is not won back
 
 static size_t sv_forward_floats(const SvPlan& p, int64_t n_bins) {
   const size_t views = (size_t)p.slices * n_bins * p.nb, split = (size_t)p.ranges * p.maxp * 2;
@@ -537,12 +538,13 @@ static bool sv_aligned(const T* A, int64_t lda) {
   return (lda * (int64_t)sizeof(T)) % 16 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
 }
 
+// el: bytes of a value of A; 0: the most that a plan for any type and alignment takes.
 static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap, size_t el, bool aligned) {
   const int64_t sms = num_sms();
   SvPlan p{};
   p.ldp = (int64_t)align_up((size_t)V, 8);
-  if (n_rot == 2 && el == sizeof(float) && (size_t)p.ldp * 2 * sizeof(float) <= kSvSplitSmem &&
-      n_bins * V * (int64_t)el >= kSvSplitBytes) {
+  if (n_rot == 2 && el != sizeof(__nv_bfloat16) && (size_t)p.ldp * 2 * sizeof(float) <= kSvSplitSmem &&
+      n_bins * V * (int64_t)sizeof(float) >= kSvSplitBytes) {
     p.ranges = sms * 32;
     p.maxp = (int)((n_bins + p.ranges - 1) / p.ranges) + 2;
   }
@@ -563,7 +565,7 @@ static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap, size_
     if (slices < want) slices = want;
     if (slices > units) slices = units;
     // back: about two CTAs an SM, at least eight rows a warp
-    const int64_t tile = sv_back_cols(p.nb, el, aligned), tiles = (V + tile - 1) / tile;
+    const int64_t tile = sv_back_cols(p.nb, el ? el : sizeof(__nv_bfloat16), aligned), tiles = (V + tile - 1) / tile;
     const int64_t most = (n_bins + 63) / 64;
     int64_t chunks = (2 * sms + tiles - 1) / tiles;
     if (chunks > most) chunks = most;
@@ -584,14 +586,19 @@ static SvPlan plan_views(int64_t n_bins, int64_t V, int n_rot, size_t cap, size_
       }
       return best;
     };
-    slices = cheapest(slices, slices + 8 < units ? slices + 8 : units, [&](int64_t k) {
+    const int64_t slices_to = slices + 8 < units ? slices + 8 : units, chunks_to = chunks + 8 < most ? chunks + 8 : most;
+    if (el == 0) {
+      slices = slices_to;
+      chunks = chunks_to;
+    }
+    if (work >= kSvPlanBytes) slices = cheapest(slices, slices_to, [&](int64_t k) {
       const int64_t splits = wave / k < 1 ? 1 : (wave / k < groups ? wave / k : groups);
       const double rounds = (double)((groups + splits - 1) / splits) * (double)((k * splits + wave - 1) / wave);
       return work * rounds * (double)wave / (double)(groups * k) + turn * rounds +
              8.0 * (double)(k * n_bins * p.nb);
     });
     const int64_t slots = sms * sv_back_ctas(p.nb);
-    chunks = cheapest(chunks, chunks + 8 < most ? chunks + 8 : most, [&](int64_t k) {
+    if (work >= kSvPlanBytes) chunks = cheapest(chunks, chunks_to, [&](int64_t k) {
       // (two CTAs of three already draw the full rate: a last round of fewer takes as long as theirs)
       const int64_t full = tiles * k / slots, rest = tiles * k % slots, least = 2 * slots / 3;
       const double share = (double)(full * slots + (rest == 0 ? 0 : rest < least ? least : rest));
