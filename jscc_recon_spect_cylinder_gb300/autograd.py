@@ -104,7 +104,9 @@ class ComptonLogLik(torch.autograd.Function):
 def poisson_log_likelihood(x, sc=None, compton=None, eps=float(torch.finfo(torch.float32).tiny)):
     """L(x) of the joint data. ``sc = (sysmat, proj [B, R], rotmat, rotmat_inv)`` (rotation
     tables may be None, then R = 1); ``compton = (events, coor, sysmat, s_c)`` with s_c the
-    Compton sensitivity [V, 1] (the list-mode term's expected-count part). Differentiable in x.
+    Compton sensitivity [V, 1] (the list-mode term's expected-count part). Differentiable in x; where a
+    float32 x takes a gradient, it is computed with the value (and has no second derivative), so a value
+    alone is cheaper under torch.no_grad().
 
     The projections come from the float32 kernels; the logarithms and the sums are taken in
     float64 (a float32 sum of ~1e4 terms carries a rounding error far above what a finite

@@ -31,9 +31,11 @@
 //     accumulators alternate ("acc_full", "acc_free" mbarriers), so the tensor cores never wait;
 //   * adders (one or two groups of four warps): each warp reads its 32 TMEM lanes of one accumulator with tcgen05.ld,
 //     adds them to FP32 registers, and writes its rows at the end.
-// 4,096 x 36,000 (9 splits) and 36,000 x 4,096 by 128 columns, launch to end with a flushed L2: 95 and
-// 87 us with tiles of 128 rows and undrained sums, 81 and 72 us so (P's bytes at copy rate: 43 us);
-// by 256 columns 132 and 117 -> 101 and 89 us; by 6 columns 70 and 66 -> 72 and 66 us.
+// 4,096 x 36,000 (four or eight splits) and 36,000 x 4,096, back to back (P is more than twice the L2), with tiles
+// of 128 rows and undrained sums and so: by 128 columns 85 and 78 -> 67 and 64 us (P's bytes at copy rate:
+// 43 us); by 256 columns 127 and 114 -> 83 and 81 us; by 6 columns 56 and 52 us either way. Where one CTA's
+// chain of K steps is all there is, few columns and one split, draining costs 3% (4,096 x 36,000 by 6: 190 and
+// 196 us).
 //   Every wait is bounded (jscc_set_wait_limit) and polls a CTA abort flag. A CTA that gives
 //   up first waits, with a fixed bound of its own, for the work it already issued: the TMA
 //   loads that the MMA issuer did not consume (they still write shared memory) and the MMAs

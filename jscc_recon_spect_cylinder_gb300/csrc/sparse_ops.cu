@@ -1909,8 +1909,8 @@ constexpr int kSpSeg = 4096;
 // (qb - qa), one weight a voxel in registers (two leave one CTA an SM, 0.35 instead of 0.24 ms). The q
 // segment staged per group is the flat range of coarse voxels that the tile's taps touch. A thread whose
 // runs are not such pairs reads its taps from global memory.
-// Bound: HBM (sysmat rows) and issue. 12,288 BF16 rows of 36,000 voxels from 25 x 90: 0.24 ms (3.7 TB/s)
-// against 1.23 ms for a thread per voxel gathering q from L2; from 100 x 90: 0.247 ms (5.4 TB/s)
+// Bound: HBM (sysmat rows) and issue. 12,288 BF16 rows of 36,000 voxels from 25 x 90: 0.235 ms (3.8 TB/s)
+// against 1.23 ms for a thread per voxel gathering q from L2; from 100 x 90: 0.225 ms (5.9 TB/s)
 // against 0.266 ms for a tile per plane with two weights a voxel.
 template <typename TE>
 __global__ void __launch_bounds__(kScThreads, 2)
